@@ -29,7 +29,7 @@ struct astr_ctx {
 struct astr_scheme {
   astr_ctx* ctx = nullptr;
   HostOp h;
-  DevOp d;
+  DevColOp d[2];               // for x lines, and for y and z lines
 };
 
 // Launch shape of one pass: solve layout (S rows per lane, WPL warps per line) and TI lines
@@ -219,7 +219,7 @@ int line_call(astr_ctx* ctx, const astr_scheme* s, int dir, const double* f, con
     df_ = tf;
     dout = to;
   }
-  cudaError_t e = launch_line_api(s->d, dir, df_, fa, dout, oa, nfields, scale, ctx->stream, flags);
+  cudaError_t e = launch_line_api(s->d[dir == 0 ? 0 : 1], dir, df_, fa, dout, oa, nfields, scale, ctx->stream, flags);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "line kernel");
   if (where == ASTR_HOST) {
     if (ob >= STAGED_MIN_BYTES && host_pageable(out)) {
@@ -230,6 +230,22 @@ int line_call(astr_ctx* ctx, const astr_scheme* s, int dir, const double* f, con
     }
     CK(cudaStreamSynchronize(ctx->stream));
   }
+  return ASTR_OK;
+}
+
+// Column operators of a new scheme; takes s over on failure.
+int scheme_tables(astr_ctx* ctx, astr_scheme* s, astr_scheme** out) {
+  const int nsys = s->h.nsys();
+  if (col_rows_per_chunk(nsys, 0) == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
+  for (int k = 0; k < 2; ++k) {
+    const cudaError_t e = make_colop(s->h, col_rows_per_chunk(nsys, k), 0, s->d[k]);
+    if (e != cudaSuccess) {
+      for (DevColOp& d : s->d) free_colop(d);
+      delete s;
+      return cuda_fail(ctx, e, "scheme tables");
+    }
+  }
+  *out = s;
   return ASTR_OK;
 }
 
@@ -619,12 +635,7 @@ int astr_fd_scheme_create(astr_ctx* ctx, const char scheme[4], int ntype, int di
     delete s;
     return fail(ctx, ASTR_ERR_ARG, "scheme not defined (only 643c and 643e) or bad ntype/dim");
   }
-  Layout lay = pick_layout(s->h.nsys());
-  if (lay.S == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
-  cudaError_t e = make_devop(s->h, lay, s->d);
-  if (e != cudaSuccess) { free_devop(s->d); delete s; return cuda_fail(ctx, e, "scheme tables"); }
-  *out = s;
-  return ASTR_OK;
+  return scheme_tables(ctx, s, out);
 }
 
 int astr_filter_create(astr_ctx* ctx, int ntype, int dim, double alpha_f, double beta_halo, double beta_bound,
@@ -635,12 +646,7 @@ int astr_filter_create(astr_ctx* ctx, int ntype, int dim, double alpha_f, double
   astr_scheme* s = new astr_scheme();
   s->ctx = ctx;
   build_filter_op(s->h, ntype, dim, alpha_f, beta_halo, beta_bound, boundary_no_filter != 0);
-  Layout lay = pick_layout(s->h.nsys());
-  if (lay.S == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
-  cudaError_t e = make_devop(s->h, lay, s->d);
-  if (e != cudaSuccess) { free_devop(s->d); delete s; return cuda_fail(ctx, e, "scheme tables"); }
-  *out = s;
-  return ASTR_OK;
+  return scheme_tables(ctx, s, out);
 }
 
 int astr_flux_create(astr_ctx* ctx, int scheme, int ntype, int dim, char wind, double bfac, astr_scheme** out) {
@@ -654,18 +660,13 @@ int astr_flux_create(astr_ctx* ctx, int scheme, int ntype, int dim, char wind, d
     delete s;
     return fail(ctx, ASTR_ERR_ARG, "flux scheme not defined (only 543) or bad ntype/dim");
   }
-  Layout lay = pick_layout(s->h.nsys());
-  if (lay.S == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
-  cudaError_t e = make_devop(s->h, lay, s->d);
-  if (e != cudaSuccess) { free_devop(s->d); delete s; return cuda_fail(ctx, e, "scheme tables"); }
-  *out = s;
-  return ASTR_OK;
+  return scheme_tables(ctx, s, out);
 }
 
 int astr_scheme_destroy(astr_scheme* s) {
   const DeviceGuard dg_(s && s->ctx ? s->ctx->device : -1);
   if (!s) return ASTR_ERR_ARG;
-  free_devop(s->d);
+  for (DevColOp& d : s->d) free_colop(d);
   delete s;
   return ASTR_OK;
 }

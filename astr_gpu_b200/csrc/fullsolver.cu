@@ -718,7 +718,7 @@ struct astr_full {
   int* counter = nullptr;
   int hist_cap = 1 << 16;
   HostOp hd[3], hf[3], hfu[3], hfd[3];
-  DevOp dd[3], df[3], dfu[3], dfd[3];
+  DevColOp dd[3], df[3], dfu[3], dfd[3];
   int nstep = 0;
   double time = 0.0;
   std::vector<double> row_key;
@@ -761,7 +761,7 @@ double* view(const astr_full* fs, double* base, int full, ArrDesc& a) {
 }
 
 // out (nodes 0..N) [+]= scale * op(in) along dir for nf fields
-cudaError_t line_op(astr_full* fs, const DevOp& op, int dir, double* in, double* out, int nf, double scale, int add) {
+cudaError_t line_op(astr_full* fs, const DevColOp& op, int dir, double* in, double* out, int nf, double scale, int add) {
   ArrDesc fa, oa;
   double* fp = view(fs, in, dir, fa);
   double* op_ = view(fs, out, -1, oa);
@@ -769,7 +769,7 @@ cudaError_t line_op(astr_full* fs, const DevOp& op, int dir, double* in, double*
 }
 
 // fh (interfaces -1..N along dir, nodes 0..N elsewhere) = the compact flux of in along dir
-cudaError_t flux_op(astr_full* fs, const DevOp& op, int dir, double* in, double* out, int nf) {
+cudaError_t flux_op(astr_full* fs, const DevColOp& op, int dir, double* in, double* out, int nf) {
   ArrDesc fa, oa;
   double* fp = view(fs, in, dir, fa);
   double* op_ = view(fs, out, -1, oa);
@@ -1047,10 +1047,10 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
   for (int d = 0; d < 3; ++d) {
     build_fd_op(fs->hd[d], "643c", g.ntype[d], N[d]);
     build_filter_op(fs->hf[d], g.ntype[d], N[d], p->alfa_filter, p->beta_halo, p->beta_bound, false);
-    const Layout L = pick_layout(fs->hf[d].nsys());
-    if (L.S == 0) { delete fs; astr_ctx_set_error(ctx, "dimension too large (max 1145)"); return ASTR_ERR_UNSUPPORTED; }
-    if (make_devop(fs->hd[d], pick_layout(fs->hd[d].nsys()), fs->dd[d]) != cudaSuccess ||
-        make_devop(fs->hf[d], L, fs->df[d]) != cudaSuccess) {
+    const int L = col_rows_per_chunk(fs->hf[d].nsys(), d);
+    if (L == 0) { delete fs; astr_ctx_set_error(ctx, "dimension too large (max 1145)"); return ASTR_ERR_UNSUPPORTED; }
+    if (make_colop(fs->hd[d], col_rows_per_chunk(fs->hd[d].nsys(), d), 0, fs->dd[d]) != cudaSuccess ||
+        make_colop(fs->hf[d], L, 0, fs->df[d]) != cudaSuccess) {
       astr_full_destroy(fs);
       astr_ctx_set_error(ctx, "scheme tables");
       return ASTR_ERR_CUDA;
@@ -1058,8 +1058,8 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
     if (upwind) {
       build_flux_op(fs->hfu[d], 543, g.ntype[d], N[d], 1, p->bfacmpld);
       build_flux_op(fs->hfd[d], 543, g.ntype[d], N[d], -1, p->bfacmpld);
-      const Layout Lf = pick_layout(fs->hfu[d].nsys());
-      if (make_devop(fs->hfu[d], Lf, fs->dfu[d]) != cudaSuccess || make_devop(fs->hfd[d], Lf, fs->dfd[d]) != cudaSuccess) {
+      const int Lf = col_rows_per_chunk(fs->hfu[d].nsys(), d);
+      if (make_colop(fs->hfu[d], Lf, 0, fs->dfu[d]) != cudaSuccess || make_colop(fs->hfd[d], Lf, 0, fs->dfd[d]) != cudaSuccess) {
         astr_full_destroy(fs);
         astr_ctx_set_error(ctx, "scheme tables");
         return ASTR_ERR_CUDA;
@@ -1101,7 +1101,7 @@ int astr_full_destroy(astr_full* fs) {
   const OnDev on(astr_ctx_device(fs->ctx));
   cudaStreamSynchronize(astr_ctx_stream(fs->ctx));
   for (int d = 0; d < 3; ++d) {
-    free_devop(fs->dd[d]); free_devop(fs->df[d]); free_devop(fs->dfu[d]); free_devop(fs->dfd[d]);
+    free_colop(fs->dd[d]); free_colop(fs->df[d]); free_colop(fs->dfu[d]); free_colop(fs->dfd[d]);
   }
   if (fs->buf) cudaFree(fs->buf);
   if (fs->partials) cudaFree(fs->partials);

@@ -5,6 +5,7 @@
 #include <string>
 #include <vector>
 
+#include "colsolve.cuh"
 #include "ops.cuh"
 
 namespace astr {
@@ -43,6 +44,27 @@ cudaError_t make_devop(const HostOp& h, Layout lay, DevOp& out);
 void fill_lineop(const HostOp& h, LineOp& o);
 void free_devop(DevOp& d);
 
+// Device-resident column operator (colsolve.cuh): S rows per chunk.
+constexpr int COL_MAXS = 37;
+struct DevColOp {
+  LineOp line{};   // the right-hand side's coefficients (no lane tables)
+  ColOp op{};
+  double* dtab = nullptr;
+  int S = 0;
+  double k1 = 0.0, k2 = 0.0, k3 = 0.0, pf[COL_MAXS] = {0}, qb[COL_MAXS] = {0};
+  template <int SS>
+  ColConst<SS> consts() const {
+    ColConst<SS> c;
+    c.k1 = k1; c.k2 = k2; c.k3 = k3;
+    for (int t = 0; t < SS; ++t) { c.pf[t] = pf[t]; c.qb[t] = qb[t]; }
+    return c;
+  }
+};
+// Rows per chunk for a system of nsys rows along dir (0: too long), and the operator itself.
+int col_rows_per_chunk(int nsys, int dir);
+cudaError_t make_colop(const HostOp& h, int S, int pad, DevColOp& out);
+void free_colop(DevColOp& d);
+
 // Tile line pitch (doubles) for TI lines of dim+1 nodes plus halos, chosen so that line-fastest
 // shared-memory accesses of a warp are free of bank conflicts.
 // Tile line pitch for lines of dim + 1 nodes, TI lines per tile, S rows per lane (schemes.cu).
@@ -53,7 +75,7 @@ struct ArrDesc { int64_t s[3]; int64_t lb[3]; int64_t n[3]; int64_t fs; };
 // flags: LINE_ADD accumulates into out (out += result) instead of storing; LINE_DIFF (interface
 // flux only) writes scale * (fh(n) - fh(n-1)) at nodes 0..dim instead of fh(-1..dim).
 enum { LINE_ADD = 1, LINE_DIFF = 2 };
-cudaError_t launch_line_api(const DevOp& op, int dir, const double* f, const ArrDesc& fa, double* out,
+cudaError_t launch_line_api(const DevColOp& op, int dir, const double* f, const ArrDesc& fa, double* out,
                             const ArrDesc& oa, int nfields, double scale, cudaStream_t st, int flags = 0);
 
 // Flow-field checkpoints (checkpoint.cu): q(n, 5) <-> the file's ro, u1, u2, u3, p, t (6 fields of

@@ -222,41 +222,15 @@ __device__ __forceinline__ void fill_window(double (&w)[W], int n0, int dim, Get
 template <class Get>
 __host__ __device__ __forceinline__ bool filter_special(const LineOp& op, int r, Get f, double& out);
 
-// Compact interface-flux closure rows, compact_flux_rhs (flux.F90:188-230): 3rd-order rows at
-// physical ends, the explicit 6th-order central interface value elsewhere. Row r is interface
-// j = r - ext_lo (between nodes j and j + 1).
-template <class Get>
-__host__ __device__ __forceinline__ bool flux_special(const LineOp& op, int r, Get f, double& out) {
-  const int j = r - op.ext_lo;
-  auto central = [&]() {
-    const double var1 = f(j) + f(j + 1), var2 = f(j - 1) + f(j + 2), var3 = f(j - 2) + f(j + 3);
-    return (37.0 / 60.0) * var1 - (2.0 / 15.0) * var2 + (1.0 / 60.0) * var3;
-  };
-  if (r == 0) {
-    out = op.left_phys ? 2.5 * f(j + 1) + 0.5 * f(j + 2) : central();
-    return true;
-  }
-  if (r == 1 && op.left_phys) { out = 0.75 * f(j) + 0.75 * f(j + 1); return true; }
-  if (r == op.nsys - 1) {
-    out = op.right_phys ? 2.5 * f(j) + 0.5 * f(j - 1) : central();
-    return true;
-  }
-  if (r == op.nsys - 2 && op.right_phys) { out = 0.75 * f(j + 1) + 0.75 * f(j); return true; }
-  return false;
-}
-
-// RHS value of closure row r (derivative or filter; with FLUX also the interface flux, which only
-// the line operators take, so that the fused passes compile without its branch), for the
-// precomputed closure table.
+// RHS value of closure row r, for the precomputed closure table.
 // KIND >= 0 fixes the operator kind at compile time (a pass that only differentiates then
 // carries no filter closure code).
-template <bool FLUX = false, int KIND = -1, class Get>
+template <int KIND = -1, class Get>
 __device__ __forceinline__ double special_value(const LineOp& op, int r, Get f) {
   double s = 0.0;
   if (KIND == OP_DERIV) deriv_special(op, r, f, s);
   else if (KIND == OP_FILTER) filter_special(op, r, f, s);
   else if (op.kind == OP_FILTER) filter_special(op, r, f, s);
-  else if (FLUX && op.kind == OP_FLUX) flux_special(op, r, f, s);
   else deriv_special(op, r, f, s);
   return s;
 }
@@ -287,43 +261,6 @@ __device__ __forceinline__ void rhs_deriv(double (&v)[S], const LineOp& op, int 
   fill_window<S + 4, S>(w, r0 - op.ext_lo - 2, op.dim, f);
   stencil_deriv<S>(v, w);
   apply_specials<S>(v, op, r0, sp);
-}
-
-// Interior rows of the compact interface flux (flux.F90:241-253), in the reference's order of
-// the four products for each wind; window w[t] = f(n0 - 1 + t), n0 = interface of the first row.
-template <int S, class Get>
-__device__ __forceinline__ void rhs_flux(double (&v)[S], const LineOp& op, int seg, Get f, const double* sp) {
-  const int r0 = seg * S;
-  double w[S + 3];
-  fill_window<S + 3, S>(w, r0 - op.ext_lo - 1, op.dim, f);
-  if (op.wind > 0) {
-#pragma unroll
-    for (int t = 0; t < S; ++t)
-      v[t] = op.cfl[0] * w[t] + op.cfl[1] * w[t + 1] + op.cfl[2] * w[t + 2] + op.cfl[3] * w[t + 3];
-  } else {
-#pragma unroll
-    for (int t = 0; t < S; ++t)
-      v[t] = op.cfl[0] * w[t + 3] + op.cfl[1] * w[t + 2] + op.cfl[2] * w[t + 1] + op.cfl[3] * w[t];
-  }
-  apply_specials<S>(v, op, r0, sp);
-}
-
-// Explicit 6th-order derivative with its closures (diff6ec, derivative.F90:350-413); rows are
-// nodes 0..dim (no solve).
-template <class Get>
-__device__ __forceinline__ double explicit_row(const LineOp& op, int i, Get v) {
-  const int dim = op.dim;
-  if (op.left_phys) {
-    if (i == 0) return -0.5 * v(2) + 2.0 * v(1) - 1.5 * v(0);
-    if (i == 1) return 0.5 * (v(2) - v(0));
-    if (i == 2) return (2.0 / 3.0) * (v(3) - v(1)) - (1.0 / 12.0) * (v(4) - v(0));
-  }
-  if (op.right_phys) {
-    if (i == dim - 2) return (2.0 / 3.0) * (v(dim - 1) - v(dim - 3)) - (1.0 / 12.0) * (v(dim) - v(dim - 4));
-    if (i == dim - 1) return 0.5 * (v(dim) - v(dim - 2));
-    if (i == dim) return 0.5 * v(dim - 2) - 2.0 * v(dim - 1) + 1.5 * v(dim);
-  }
-  return 0.75 * (v(i + 1) - v(i - 1)) - 0.15 * (v(i + 2) - v(i - 2)) + (1.0 / 60.0) * (v(i + 3) - v(i - 3));
 }
 
 // Compact filter closure rows, filter.F90:176-269. Returns false for interior rows.

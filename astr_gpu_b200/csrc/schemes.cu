@@ -5,6 +5,7 @@
 //   filter_coefficient_cal      src/filter.F90:299-432
 //   compact_flux_initiate       src/flux.F90:32-112
 //   tridiagonal_thomas_proprocess src/commfunc.F90:752-774
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -302,6 +303,85 @@ cudaError_t make_devop(const HostOp& h, Layout lay, DevOp& out) {
 }
 
 void free_devop(DevOp& d) {
+  if (d.dtab) cudaFree(d.dtab);
+  d.dtab = nullptr;
+}
+
+// Measured on a B200 (derivative / filter, GB/s of read + written nodes; lines of 32 adjacent in x
+// per CTA along y): 256 nodes 33 rows 5400 / 4160, 17 rows 3570 / 3050; 128 nodes 33 rows 4135 /
+// 2876, 17 rows 3465 / 2892; 64 nodes 17 rows 2055 / 1488, 33 rows 1707 / 1486. Along x (16 lines
+// through shared memory) 128 nodes 33 rows 2960 / 2142, 17 rows 2739 / 2410; 256 nodes 33 rows
+// 3540 / 3130, 17 rows 3094 / 2741.
+int col_rows_per_chunk(int nsys, int dir) {
+  if (nsys < 15) return 3;
+  if (nsys < 18) return 5;
+  if (nsys <= 45) return 9;
+  if (nsys <= (dir == 0 ? 176 : 90)) return 17;
+  if (nsys <= 1056) return 33;
+  if (nsys <= 1152) return 37;
+  return 0;
+}
+
+// The column solve's view of the system with `pad` identity rows before and after it (pad > 0
+// embeds an operator in the chunks of one with a longer system).
+cudaError_t make_colop(const HostOp& h, int S, int pad, DevColOp& out) {
+  fill_lineop(h, out.line);
+  out.S = S;
+  const int n0 = h.nsys(), nsys = n0 + 2 * pad;
+  const int nch = std::max(3, (nsys + S - 1) / S);
+  if (nsys < 2 * S) return cudaErrorInvalidValue;
+  ColOp& o = out.op;
+  o.nch = nch;
+  o.rag = nch / 2;
+  o.nv = nsys - (nch - 1) * S;
+  o.n_first = h.first_node - pad;
+  if (h.kind == OP_EXPLICIT) return cudaSuccess;   // rows but no system
+  const size_t rows = (size_t)nch * S;
+  std::vector<double> t(rows * 6 + 2 * (size_t)nch, 0.0);
+  for (int c = 0; c < nch; ++c) {
+    double p = 1.0, q = 1.0;
+    double* tc = t.data() + (size_t)c * S * 6;
+    for (int k = 0; k < S; ++k) {
+      double e1, e2, e3;
+      const int r = c * S + k - (c > o.rag ? S - o.nv : 0) - pad;   // row of the operator's own system
+      if (c == o.rag && k >= o.nv) { e1 = -1.0; e2 = 0.0; e3 = -1.0; }   // left over: passes the carries on
+      else if (r < 0 || r >= n0) { e1 = 0.0; e2 = 1.0; e3 = 0.0; }       // identity row
+      else {
+        e1 = (r == n0 - 1) ? 0.0 : h.ac1[r];   // back substitution starts at the last row
+        e2 = (r == 0) ? 1.0 : h.ac2[r];        // the first row of the forward sweep is untouched
+        e3 = (r == 0) ? 0.0 : h.ac3[r];
+      }
+      tc[6 * k] = e2;
+      tc[6 * k + 1] = e3;
+      p *= -e3;
+      tc[6 * k + 2] = p;
+      tc[6 * k + 3] = e1;
+    }
+    for (int k = S - 1; k >= 0; --k) { q *= -tc[6 * k + 3]; tc[6 * k + 4] = q; }
+    t[rows * 6 + c] = p;
+    t[rows * 6 + nch + c] = q;
+  }
+  // chunks whose columns are bitwise those of the last full interior chunk
+  const int ref = nch - 2 == o.rag ? nch - 3 : nch - 2;
+  auto same = [&](int c) {
+    return std::memcmp(t.data() + (size_t)c * S * 6, t.data() + (size_t)ref * S * 6, (size_t)S * 6 * sizeof(double)) == 0;
+  };
+  bool flat = ref >= 0 && ref != o.rag;   // one coefficient set through the whole chunk
+  const double* tr = t.data() + (size_t)ref * S * 6;
+  for (int k = 1; k < S && flat; ++k) flat = tr[6 * k] == tr[0] && tr[6 * k + 1] == tr[1] && tr[6 * k + 3] == tr[3];
+  o.c_hi = flat ? nch - 1 : 0;
+  o.c_lo = o.c_hi;
+  while (o.c_lo > 0 && (o.c_lo - 1 == o.rag || same(o.c_lo - 1))) --o.c_lo;
+  for (int k = 0; k < S && S <= COL_MAXS; ++k) { out.pf[k] = tr[6 * k + 2]; out.qb[k] = tr[6 * k + 4]; }
+  out.k2 = tr[0]; out.k3 = tr[1]; out.k1 = tr[3];
+  cudaError_t e = cudaMalloc(&out.dtab, t.size() * sizeof(double));
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpy(out.dtab, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice);
+  o.tab = out.dtab;
+  return e;
+}
+
+void free_colop(DevColOp& d) {
   if (d.dtab) cudaFree(d.dtab);
   d.dtab = nullptr;
 }

@@ -342,7 +342,7 @@ __device__ __forceinline__ void compute_specials(const LineOp& op, int TI, doubl
     const bool lo = j < NSP;
     if (lo ? (j >= op.spec_lo) : (j - NSP >= op.spec_hi)) continue;
     const int r = lo ? j : op.nsys - op.spec_hi + (j - NSP);
-    sp[(l * ns + k) * per + j] = special_value<false, KIND>(op, r, [&](int n) { return getk(l, k, n); });
+    sp[(l * ns + k) * per + j] = special_value<KIND>(op, r, [&](int n) { return getk(l, k, n); });
   }
 }
 
