@@ -1,5 +1,6 @@
 // C-ABI implementation (include/astr_b200.h): contexts, schemes, the solver state, and the
 // orchestration of the RK3 step as fused passes (one CUDA graph per step).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -13,6 +14,7 @@
 #include "../../include/astr_b200.h"
 #include "internal.h"
 #include "tgv.cuh"
+#include "tgv_cols.h"
 #include "adjoint.cuh"
 
 using namespace astr;
@@ -56,9 +58,11 @@ struct astr_state {
   HostOp hd[3], hf[3];                     // derivative and filter operators per direction
   std::map<int, std::pair<DevOp, DevOp>> ops;   // lane tables per (direction, layout)
   PassCfg cfg[NCFG];                       // launch shape of every pass
+  ColDir col[3];                           // column operators along y and z (x unused)
+  bool use_col[NCFG] = {true, true, false, true, true, false, true};   // passes run as column solves
   bool autotune = true, tuned = false;
   bool pending = false;       // filter along DIR_A of the last stage not yet applied
-  bool split_fa = false;      // that filter as its own streaming pass (else fused into pass A)
+  bool split_fa = true;       // that filter as its own pass (else fused into pass A)
   int nstep = 0;
   double time = 0.0;
   std::vector<double> row_key;  // (nstep, time) per history row
@@ -237,13 +241,12 @@ int line_call(astr_ctx* ctx, const astr_scheme* s, int dir, const double* f, con
 int scheme_tables(astr_ctx* ctx, astr_scheme* s, astr_scheme** out) {
   const int nsys = s->h.nsys();
   if (col_rows_per_chunk(nsys, 0) == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
-  for (int k = 0; k < 2; ++k) {
-    const cudaError_t e = make_colop(s->h, col_rows_per_chunk(nsys, k), 0, s->d[k]);
-    if (e != cudaSuccess) {
-      for (DevColOp& d : s->d) free_colop(d);
-      delete s;
-      return cuda_fail(ctx, e, "scheme tables");
-    }
+  const ColSpec specs[2] = {{&s->h, col_rows_per_chunk(nsys, 0), 0, &s->d[0]}, {&s->h, col_rows_per_chunk(nsys, 1), 0, &s->d[1]}};
+  const cudaError_t e = make_colops(specs, 2);
+  if (e != cudaSuccess) {
+    free_colop(s->d[0]);
+    delete s;
+    return cuda_fail(ctx, e, "scheme tables");
   }
   *out = s;
   return ASTR_OK;
@@ -266,15 +269,19 @@ int diag_parts(astr_state* st) {
   return (int)(((st->g.N[o1] + 1 + ti - 1) / ti) * (int64_t)(st->g.N[o2] + 1));
 }
 
-PassArgs base_args(astr_state* st, int id) {
+// Arguments of pass `id`; lane: with the tables of its lane-scan kernel (which the batched ensemble
+// passes always run).
+PassArgs base_args(astr_state* st, int id, bool lane) {
   const PassCfg& pc = st->cfg[id];
   const int dir = CFG_DIR[id];
-  auto& o = get_ops(st, dir, pc.S, pc.WPL);
   PassArgs a{};
   a.g = st->g;
   a.th = st->th;
-  a.opd = o.first.op;
-  a.opf = o.second.op;
+  if (lane) {
+    auto& o = get_ops(st, dir, pc.S, pc.WPL);
+    a.opd = o.first.op;
+    a.opf = o.second.op;
+  }
   a.dir = dir;
   a.dA = DIR_A; a.dB = DIR_B; a.dC = DIR_C;
   a.TI = pc.TI;
@@ -286,6 +293,8 @@ PassArgs base_args(astr_state* st, int id) {
   a.err = st->err;
   return a;
 }
+
+PassArgs base_args(astr_state* st, int id) { return base_args(st, id, !st->use_col[id]); }
 
 // Optional per-pass event timing (astr_pass_timings); null in normal runs.
 struct PassTimer {
@@ -302,7 +311,19 @@ cudaError_t run_pass(astr_state* st, int id, PassArgs& a) {
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st->ctx->stream);
   }
-  cudaError_t e = launch_pass(pass, a, st->cfg[id].S, st->cfg[id].WPL, st->ctx->stream);
+  const ColDir& cd = st->col[a.dir];
+  cudaStream_t sm = st->ctx->stream;
+  cudaError_t e;
+  if (!st->use_col[id]) e = launch_pass(pass, a, st->cfg[id].S, st->cfg[id].WPL, sm);
+  else if (id == CFG_FA) e = launch_col_pass(0, a, nullptr, cd, sm);
+  else if (id == CFG_VA) e = launch_col_pass(2, a, st->VF, cd, sm);
+  else if (id == CFG_VB) e = launch_col_pass(a.mode == 0 ? 2 : 3, a, st->VF + 5 * st->g.fs, cd, sm);
+  else {
+    // the gradients along y and z differentiate the primitives that the first of them stores in VF's
+    // first four fields (free until pass C fills VF)
+    e = id == CFG_A || !st->use_col[CFG_A] ? launch_prims(a, st->VF, sm) : cudaSuccess;
+    if (e == cudaSuccess) e = launch_col_pass(1, a, st->VF, cd, sm);
+  }
   if (g_timer) {
     cudaEventRecord(e1, st->ctx->stream);
     g_timer->ev.push_back(e0);
@@ -495,6 +516,8 @@ cudaError_t autotune(astr_state* st) {
   float tbest[NCFG], tfused = 1e30f;
   PassCfg fusedc = st->cfg[CFG_A];
   for (int id = 0; id < NCFG; ++id) {
+    tbest[id] = 0.0f;
+    if (st->use_col[id]) continue;
     const int dir = CFG_DIR[id], pass = CFG_PASS[id];
     const int nsys = st->hf[dir].nsys();
     const int dim = st->g.N[dir];
@@ -556,8 +579,10 @@ cudaError_t autotune(astr_state* st) {
     st->cfg[id] = bestc;
     tbest[id] = best;
   }
-  st->split_fa = filt && tbest[CFG_A] + tbest[CFG_FA] < tfused;
-  if (filt && !st->split_fa) st->cfg[CFG_A] = fusedc;
+  if (!st->use_col[CFG_A]) {
+    st->split_fa = filt && tbest[CFG_A] + tbest[CFG_FA] < tfused;
+    if (filt && !st->split_fa) st->cfg[CFG_A] = fusedc;
+  }
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
   e = cudaMemsetAsync(st->err, 0, sizeof(int), sm);
@@ -666,7 +691,7 @@ int astr_flux_create(astr_ctx* ctx, int scheme, int ntype, int dim, char wind, d
 int astr_scheme_destroy(astr_scheme* s) {
   const DeviceGuard dg_(s && s->ctx ? s->ctx->device : -1);
   if (!s) return ASTR_ERR_ARG;
-  for (DevColOp& d : s->d) free_colop(d);
+  free_colop(s->d[0]);
   delete s;
   return ASTR_OK;
 }
@@ -766,12 +791,14 @@ int astr_state_create(astr_ctx* ctx, const astr_params* p, astr_state** out) {
     c.TI = pick_ti(pass_tiles(CFG_PASS[id]), N[d], L.WPL, L.S);
     c.LP = tile_pitch(N[d], c.TI, c.S);
   }
+  const cudaError_t ec = make_coldirs(st->hd, st->hf, st->col);
+  if (ec != cudaSuccess) { astr_state_destroy(st); return cuda_fail(ctx, ec, "column operators"); }
   // a small box gains nothing from tuning
   st->autotune = (N[0] + 1) * (int64_t)(N[1] + 1) * (N[2] + 1) >= 100 * 100 * 100;
   // 33 fields: Q0(5) Q1(5) R(5) DA(4) DB(4) VF(10: the combined fluxes along A and along B)
   const size_t nf = 33;
   cudaError_t e = cudaMalloc(&st->buf, nf * (size_t)st->g.fs * sizeof(double));
-  if (e != cudaSuccess) { delete st; return fail(ctx, ASTR_ERR_NOMEM, "state allocation"); }
+  if (e != cudaSuccess) { astr_state_destroy(st); return fail(ctx, ASTR_ERR_NOMEM, "state allocation"); }
   cudaMemsetAsync(st->buf, 0, nf * (size_t)st->g.fs * sizeof(double), ctx->stream);
   st->Q0 = st->buf;
   st->Q1 = st->Q0 + 5 * st->g.fs;
@@ -799,6 +826,7 @@ int astr_state_destroy(astr_state* st) {
   if (!st) return ASTR_ERR_ARG;
   drop_graphs(st);
   for (auto& kv : st->ops) { free_devop(kv.second.first); free_devop(kv.second.second); }
+  free_coldirs(st->col);
   if (st->buf) cudaFree(st->buf);
   if (st->partials) cudaFree(st->partials);
   if (st->hist) cudaFree(st->hist);
@@ -945,6 +973,11 @@ int astr_state_autotune(astr_state* st, int on) {
 int astr_state_launch_shapes(astr_state* st, int shapes[42]) {
   if (!st || !shapes) return ASTR_ERR_ARG;
   for (int id = 0; id < NCFG; ++id) {
+    if (st->use_col[id]) {
+      const int col[6] = {st->col[CFG_DIR[id]].d.S, 0, col_lines(st->col[CFG_DIR[id]]), 0, 1, 1};
+      std::copy(col, col + 6, shapes + 6 * id);
+      continue;
+    }
     shapes[6 * id] = st->cfg[id].S;
     shapes[6 * id + 1] = st->cfg[id].WPL;
     shapes[6 * id + 2] = st->cfg[id].TI;
@@ -979,6 +1012,7 @@ int astr_state_set_launch_shape(astr_state* st, int pass, int S, int WPL, int TI
   PassCfg c;
   c.S = S; c.WPL = WPL; c.TI = TI; c.LP = tile_pitch(st->g.N[dir], TI, S); c.LPW = LPW; c.FPS = FPS;
   st->cfg[pass] = c;
+  st->use_col[pass] = false;
   st->autotune = false;
   drop_graphs(st);
   return ASTR_OK;
@@ -988,6 +1022,7 @@ int astr_state_split_filter(astr_state* st, int on) {
   const DeviceGuard dg_(st ? st->ctx->device : -1);
   if (!st) return ASTR_ERR_ARG;
   st->split_fa = on != 0;
+  if (!on) st->use_col[CFG_A] = false;   // the fused form is the lane-scan pass
   st->autotune = false;
   drop_graphs(st);
   return ASTR_OK;
@@ -1196,7 +1231,7 @@ int ens_build(astr_ensemble* e) {
             PassCfg c;
             c.S = g.S; c.WPL = g.WPL; c.TI = g.TI[id]; c.LP = tile_pitch(st->g.N[dir], c.TI, g.S);
             st->cfg[id] = c;
-            PassArgs a = base_args(st, id);
+            PassArgs a = base_args(st, id, true);
             double* qin = (s == 0) ? st->Q0 : st->Q1;
             double* qout = (s == 2) ? st->Q0 : st->Q1;
             const int filt = st->p.filter_on;
@@ -1298,7 +1333,7 @@ int ens_tune(astr_ensemble* e, bool timed) {
           PassCfg c;
           c.S = g.S; c.WPL = g.WPL; c.TI = ti; c.LP = tile_pitch(st->g.N[dir], ti, g.S);
           st->cfg[id] = c;
-          PassArgs a = base_args(st, id);
+          PassArgs a = base_args(st, id, true);
           st->cfg[id] = saved;
           a.q = st->Q1; a.D = st->DA; a.DA = st->DA; a.DB = st->DB; a.partials = nullptr;
           // stage 2-3 form of the update: q (scratch) and qsave (live state, only read) distinct

@@ -1044,27 +1044,29 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
                             "periodic directions only on one rank");
     return ASTR_ERR_UNSUPPORTED;
   }
+  std::vector<ColSpec> specs;
   for (int d = 0; d < 3; ++d) {
     build_fd_op(fs->hd[d], "643c", g.ntype[d], N[d]);
     build_filter_op(fs->hf[d], g.ntype[d], N[d], p->alfa_filter, p->beta_halo, p->beta_bound, false);
-    const int L = col_rows_per_chunk(fs->hf[d].nsys(), d);
-    if (L == 0) { delete fs; astr_ctx_set_error(ctx, "dimension too large (max 1145)"); return ASTR_ERR_UNSUPPORTED; }
-    if (make_colop(fs->hd[d], col_rows_per_chunk(fs->hd[d].nsys(), d), 0, fs->dd[d]) != cudaSuccess ||
-        make_colop(fs->hf[d], L, 0, fs->df[d]) != cudaSuccess) {
-      astr_full_destroy(fs);
-      astr_ctx_set_error(ctx, "scheme tables");
-      return ASTR_ERR_CUDA;
-    }
+    auto add = [&](HostOp& h, DevColOp& o) { specs.push_back(ColSpec{&h, col_rows_per_chunk(h.nsys(), d), 0, &o}); };
+    add(fs->hd[d], fs->dd[d]);
+    add(fs->hf[d], fs->df[d]);
     if (upwind) {
       build_flux_op(fs->hfu[d], 543, g.ntype[d], N[d], 1, p->bfacmpld);
       build_flux_op(fs->hfd[d], 543, g.ntype[d], N[d], -1, p->bfacmpld);
-      const int Lf = col_rows_per_chunk(fs->hfu[d].nsys(), d);
-      if (make_colop(fs->hfu[d], Lf, 0, fs->dfu[d]) != cudaSuccess || make_colop(fs->hfd[d], Lf, 0, fs->dfd[d]) != cudaSuccess) {
-        astr_full_destroy(fs);
-        astr_ctx_set_error(ctx, "scheme tables");
-        return ASTR_ERR_CUDA;
-      }
+      add(fs->hfu[d], fs->dfu[d]);
+      add(fs->hfd[d], fs->dfd[d]);
     }
+    if (col_rows_per_chunk(fs->hf[d].nsys(), d) == 0) {
+      delete fs;
+      astr_ctx_set_error(ctx, "dimension too large (max 1145)");
+      return ASTR_ERR_UNSUPPORTED;
+    }
+  }
+  if (make_colops(specs.data(), (int)specs.size()) != cudaSuccess) {
+    astr_full_destroy(fs);
+    astr_ctx_set_error(ctx, "scheme tables");
+    return ASTR_ERR_CUDA;
   }
   // q(5) qt(5) rho vel(3) prs tmp qsave(5) qrhs(5) dvel(9) dtmp(3) sigma(6) qflux(3) work(5)
   // [+ f+ f- fh+ fh- (20), ssf and lshock (2) for the upwind convection]
@@ -1100,9 +1102,7 @@ int astr_full_destroy(astr_full* fs) {
   if (!fs) return ASTR_ERR_ARG;
   const OnDev on(astr_ctx_device(fs->ctx));
   cudaStreamSynchronize(astr_ctx_stream(fs->ctx));
-  for (int d = 0; d < 3; ++d) {
-    free_colop(fs->dd[d]); free_colop(fs->df[d]); free_colop(fs->dfu[d]); free_colop(fs->dfd[d]);
-  }
+  free_colop(fs->dd[0]);
   if (fs->buf) cudaFree(fs->buf);
   if (fs->partials) cudaFree(fs->partials);
   if (fs->hist) cudaFree(fs->hist);

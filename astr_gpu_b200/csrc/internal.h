@@ -51,19 +51,26 @@ struct DevColOp {
   ColOp op{};
   double* dtab = nullptr;
   int S = 0;
-  double k1 = 0.0, k2 = 0.0, k3 = 0.0, pf[COL_MAXS] = {0}, qb[COL_MAXS] = {0};
+  double k1 = 0.0, k2 = 1.0, k3 = 0.0, pf[COL_MAXS] = {0}, qb[COL_MAXS] = {0};
   template <int SS>
   ColConst<SS> consts() const {
     ColConst<SS> c;
-    c.k1 = k1; c.k2 = k2; c.k3 = k3;
+    c.k1 = k1; c.k3 = k3;
     for (int t = 0; t < SS; ++t) { c.pf[t] = pf[t]; c.qb[t] = qb[t]; }
     return c;
   }
 };
 // Rows per chunk for a system of nsys rows along dir (0: too long), and the operator itself.
 int col_rows_per_chunk(int nsys, int dir);
-cudaError_t make_colop(const HostOp& h, int S, int pad, DevColOp& out);
+struct ColSpec {
+  const HostOp* h;
+  int S, pad;      // rows per chunk, identity rows around the system
+  DevColOp* out;
+};
+cudaError_t make_colops(const ColSpec* specs, int n);   // one allocation, freed with the first
 void free_colop(DevColOp& d);
+// Right-hand side weights for an output scaled by `scale`.
+ColWeights col_weights(const DevColOp& d, double scale);
 
 // Tile line pitch (doubles) for TI lines of dim+1 nodes plus halos, chosen so that line-fastest
 // shared-memory accesses of a warp are free of bank conflicts.

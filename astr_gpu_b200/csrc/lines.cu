@@ -49,12 +49,12 @@ __device__ __forceinline__ void window(double (&w)[W], const double* src, int64_
 }
 
 template <int S, int KIND>
-__device__ __forceinline__ void line_rhs(double (&v)[S], const double (&w)[S + Win<KIND>::EXTRA], const LineOp& op,
-                                         const ColOp& co, int c) {
-  if constexpr (KIND == OP_DERIV) col_rhs_deriv<S>(v, w, c, co.nch, op.left_phys, op.right_phys);
+__device__ __forceinline__ void line_rhs(double (&v)[S], const double (&w)[S + Win<KIND>::EXTRA], const ColWeights& k,
+                                         const LineOp& op, const ColOp& co, int c) {
+  if constexpr (KIND == OP_DERIV) col_rhs_deriv<S>(v, w, k, c, co.nch, op.left_phys, op.right_phys);
   else if constexpr (KIND == OP_EXPLICIT) col_explicit<S>(v, w, c, co.nch, op.left_phys, op.right_phys);
-  else if constexpr (KIND == OP_FILTER) col_rhs_filter<S>(v, w, op, c, co.nch);
-  else col_rhs_flux<S>(v, w, op, c, co.nch);
+  else if constexpr (KIND == OP_FILTER) col_rhs_filter<S>(v, w, k, op, c, co.nch);
+  else col_rhs_flux<S>(v, w, k, op, c, co.nch);
   col_zero_ragged<S>(v, co, c);
 }
 
@@ -64,6 +64,7 @@ struct LineArgs {
   ArrDesc fa, oa;
   int dir, flags;
   double scale;
+  ColWeights k;
 };
 
 }  // namespace
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 256, S >= 17 ? 1 : 2)
   double* exf = sm;
   double* exb = sm + co.nch * LW;
   const int dir = a.dir, o2 = dir == 2 ? 1 : 2;
-  const int l = threadIdx.x % LW, c = threadIdx.x / LW;
+  const int l = threadIdx.x % LW, c = col_chunk(co, threadIdx.x / LW);
   // the line: tiles of LW lines along x per index of the third axis, or (blockIdx.y unused) of LW
   // consecutive lines of the flattened (x, third axis) plane
   int64_t x1 = (int64_t)blockIdx.x * LW + l, x2 = blockIdx.y;
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 256, S >= 17 ? 1 : 2)
     window<W>(w, src, fd, n0 - Win<KIND>::LO, lo, hi);
     // physical-boundary reset ff(0)=f(0), ff(dim)=f(dim) of compact_filter (filter.F90:141-142)
     if (KIND == OP_FILTER) keep = c == 0 ? w[5] : w[S + 4];
-    line_rhs<S, KIND>(v, w, op, co, c);
+    line_rhs<S, KIND>(v, w, a.k, op, co, c);
   }
   if (KIND == OP_EXPLICIT) __syncthreads();   // every window is read before the first store
   else col_solve<S, LW>(v, co, k, c, l, act, exf, exb);
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 256, S >= 17 ? 1 : 2)
     __syncthreads();
     if (act) {
       double prev = 0.0;
-      if (c > 0) prev = (c - 1 == co.rag && co.nv == 0) ? exf[(c - 2) * LW + l] : exf[(c - 1) * LW + l];
+      if (c > 0) prev = (c == 2 && co.nv == 0) ? exf[l] : exf[(c - 1) * LW + l];
 #pragma unroll
       for (int t = 0; t < S; ++t) {
         const double x = v[t];
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 256, S >= 17 ? 1 : 2)
   const int64_t od = dir == 1 ? a.oa.s[1] : a.oa.s[2], oo = dir == 1 ? a.oa.s[2] : a.oa.s[1];
   const int64_t ol = dir == 1 ? a.oa.lb[1] : a.oa.lb[2];
   double* dst = a.out + (int64_t)blockIdx.z * a.oa.fs + (i2 - a.oa.lb[o2]) * oo + (i1 - a.oa.lb[0]) + (n0 - ol) * od;
-  const double sc = KIND == OP_FILTER ? 1.0 : a.scale;
+  auto res = [&](double x) { return KIND == OP_FILTER ? x : a.scale * x; };
   if (KIND == OP_FILTER) {
     if (c == 0 && op.left_phys) v[0] = keep;
     if (c == co.nch - 1 && op.right_phys) v[S - 1] = keep;
@@ -158,17 +159,17 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 256, S >= 17 ? 1 : 2)
       for (int j = 0; j < 11; ++j)
         if (t0 + j < S) {
           const int n = n0 + t0 + j;
-          if (t0 + j < nv && n >= out_lo && n <= dim) dst[(int64_t)(t0 + j) * od] = old[j] + sc * v[t0 + j];
+          if (t0 + j < nv && n >= out_lo && n <= dim) dst[(int64_t)(t0 + j) * od] = old[j] + res(v[t0 + j]);
         }
     }
   } else if (nv == S && n0 >= out_lo && n0 + S - 1 <= dim) {
 #pragma unroll
-    for (int t = 0; t < S; ++t) { *dst = sc * v[t]; dst += od; }
+    for (int t = 0; t < S; ++t) { *dst = res(v[t]); dst += od; }
   } else {
 #pragma unroll
     for (int t = 0; t < S; ++t) {
       const int n = n0 + t;
-      if (t < nv && n >= out_lo && n <= dim) *dst = sc * v[t];
+      if (t < nv && n >= out_lo && n <= dim) *dst = res(v[t]);
       dst += od;
     }
   }
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 320, S >= 17 ? 1 : 2)
   }
   cp_wait_all();
   __syncthreads();
-  const int l = threadIdx.x % LW, c = threadIdx.x / LW;
+  const int l = threadIdx.x % LW, c = col_chunk(co, threadIdx.x / LW);
   const bool act = c < co.nch;
   constexpr int W = S + Win<KIND>::EXTRA;
   const int n0 = col_node<S>(co, c);
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 320, S >= 17 ? 1 : 2)
     double w[W];
     window<W>(w, line, 1, n0 - Win<KIND>::LO, -HL, dim + HL);
     if (KIND == OP_FILTER) keep = c == 0 ? w[5] : w[S + 4];
-    line_rhs<S, KIND>(v, w, op, co, c);
+    line_rhs<S, KIND>(v, w, a.k, op, co, c);
   }
   if (KIND == OP_EXPLICIT) __syncthreads();   // every window is read before the first store
   else col_solve<S, LW>(v, co, k, c, l, act, exf, exb);
@@ -309,7 +310,7 @@ static cudaError_t launch_s(const DevColOp& op, const LineArgs& a, int nfields, 
 
 cudaError_t launch_line_api(const DevColOp& op, int dir, const double* f, const ArrDesc& fa, double* out,
                             const ArrDesc& oa, int nfields, double scale, cudaStream_t st, int flags) {
-  const LineArgs a{f, out, fa, oa, dir, flags, scale};
+  const LineArgs a{f, out, fa, oa, dir, flags, scale, col_weights(op, 1.0)};
   switch (op.S) {
     case 3: return launch_s<3>(op, a, nfields, st);
     case 5: return launch_s<5>(op, a, nfields, st);

@@ -324,7 +324,8 @@ int col_rows_per_chunk(int nsys, int dir) {
 
 // The column solve's view of the system with `pad` identity rows before and after it (pad > 0
 // embeds an operator in the chunks of one with a longer system).
-cudaError_t make_colop(const HostOp& h, int S, int pad, DevColOp& out) {
+// The host side of make_colop: everything but the device copy of the table `t`.
+static cudaError_t fill_colop(const HostOp& h, int S, int pad, DevColOp& out, std::vector<double>& t) {
   fill_lineop(h, out.line);
   out.S = S;
   const int n0 = h.nsys(), nsys = n0 + 2 * pad;
@@ -332,20 +333,20 @@ cudaError_t make_colop(const HostOp& h, int S, int pad, DevColOp& out) {
   if (nsys < 2 * S) return cudaErrorInvalidValue;
   ColOp& o = out.op;
   o.nch = nch;
-  o.rag = nch / 2;
   o.nv = nsys - (nch - 1) * S;
   o.n_first = h.first_node - pad;
+  o.c_lo = nch - 1;
   if (h.kind == OP_EXPLICIT) return cudaSuccess;   // rows but no system
   const size_t rows = (size_t)nch * S;
-  std::vector<double> t(rows * 6 + 2 * (size_t)nch, 0.0);
+  t.assign(rows * 6 + 2 * (size_t)nch, 0.0);
   for (int c = 0; c < nch; ++c) {
     double p = 1.0, q = 1.0;
     double* tc = t.data() + (size_t)c * S * 6;
     for (int k = 0; k < S; ++k) {
       double e1, e2, e3;
-      const int r = c * S + k - (c > o.rag ? S - o.nv : 0) - pad;   // row of the operator's own system
-      if (c == o.rag && k >= o.nv) { e1 = -1.0; e2 = 0.0; e3 = -1.0; }   // left over: passes the carries on
-      else if (r < 0 || r >= n0) { e1 = 0.0; e2 = 1.0; e3 = 0.0; }       // identity row
+      const int r = c * S + k - (c > 1 ? S - o.nv : 0) - pad;   // row of the operator's own system
+      if (c == 1 && k >= o.nv) { e1 = -1.0; e2 = 0.0; e3 = -1.0; }   // left over: passes the carries on
+      else if (r < 0 || r >= n0) { e1 = 0.0; e2 = 1.0; e3 = 0.0; }   // identity row
       else {
         e1 = (r == n0 - 1) ? 0.0 : h.ac1[r];   // back substitution starts at the last row
         e2 = (r == 0) ? 1.0 : h.ac2[r];        // the first row of the forward sweep is untouched
@@ -361,24 +362,58 @@ cudaError_t make_colop(const HostOp& h, int S, int pad, DevColOp& out) {
     t[rows * 6 + c] = p;
     t[rows * 6 + nch + c] = q;
   }
-  // chunks whose columns are bitwise those of the last full interior chunk
-  const int ref = nch - 2 == o.rag ? nch - 3 : nch - 2;
-  auto same = [&](int c) {
-    return std::memcmp(t.data() + (size_t)c * S * 6, t.data() + (size_t)ref * S * 6, (size_t)S * 6 * sizeof(double)) == 0;
-  };
-  bool flat = ref >= 0 && ref != o.rag;   // one coefficient set through the whole chunk
-  const double* tr = t.data() + (size_t)ref * S * 6;
+  // chunks from c_lo on have one coefficient set, bitwise that of the last chunk but one
+  const double* tr = t.data() + (size_t)(nch - 2) * S * 6;
+  bool flat = nch > 3;
   for (int k = 1; k < S && flat; ++k) flat = tr[6 * k] == tr[0] && tr[6 * k + 1] == tr[1] && tr[6 * k + 3] == tr[3];
-  o.c_hi = flat ? nch - 1 : 0;
-  o.c_lo = o.c_hi;
-  while (o.c_lo > 0 && (o.c_lo - 1 == o.rag || same(o.c_lo - 1))) --o.c_lo;
+  if (flat) {
+    o.c_lo = nch - 2;
+    while (o.c_lo > 2 && std::memcmp(t.data() + (size_t)(o.c_lo - 1) * S * 6, tr, (size_t)S * 6 * sizeof(double)) == 0) --o.c_lo;
+    if (o.c_lo % 2 == 0) ++o.c_lo;   // with the last one an even number of table chunks
+    o.c_lo = std::min(o.c_lo, nch - 1);
+  }
   for (int k = 0; k < S && S <= COL_MAXS; ++k) { out.pf[k] = tr[6 * k + 2]; out.qb[k] = tr[6 * k + 4]; }
-  out.k2 = tr[0]; out.k3 = tr[1]; out.k1 = tr[3];
-  cudaError_t e = cudaMalloc(&out.dtab, t.size() * sizeof(double));
+  out.k3 = tr[1];
+  out.k1 = tr[3];
+  out.k2 = flat ? tr[0] : 1.0;
+  for (size_t r = 0; r < rows; ++r) t[6 * r] /= out.k2;
+  return cudaSuccess;
+}
+
+// Column operators share one device table, owned by the first of them.
+cudaError_t make_colops(const ColSpec* specs, int n) {
+  std::vector<double> all;
+  std::vector<size_t> at(n);
+  for (int i = 0; i < n; ++i) {
+    std::vector<double> t;
+    const cudaError_t e = fill_colop(*specs[i].h, specs[i].S, specs[i].pad, *specs[i].out, t);
+    if (e != cudaSuccess) return e;
+    at[i] = all.size();
+    all.insert(all.end(), t.begin(), t.end());
+    all.resize((all.size() + 1) / 2 * 2);   // 16-byte rows
+  }
+  if (all.empty()) return cudaSuccess;      // explicit operators have no table
+  DevColOp& own = *specs[0].out;
+  cudaError_t e = cudaMalloc(&own.dtab, all.size() * sizeof(double));
   if (e != cudaSuccess) return e;
-  e = cudaMemcpy(out.dtab, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice);
-  o.tab = out.dtab;
+  e = cudaMemcpy(own.dtab, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice);
+  for (int i = 0; i < n; ++i) specs[i].out->op.tab = own.dtab + at[i];
   return e;
+}
+
+ColWeights col_weights(const DevColOp& d, double scale) {
+  ColWeights k{};
+  k.ks = d.k2 * scale;
+  const LineOp& o = d.line;
+  if (o.kind == OP_DERIV) {
+    k.w[0] = (7.0 / 9.0) * k.ks;
+    k.w[1] = (1.0 / 36.0) * k.ks;
+  } else if (o.kind == OP_FILTER) {
+    for (int i = 0; i < 6; ++i) k.w[i] = (i == 0 ? 2.0 : 1.0) * o.c10[i] * k.ks;
+  } else if (o.kind == OP_FLUX) {
+    for (int i = 0; i < 4; ++i) k.w[i] = o.cfl[i] * k.ks;
+  }
+  return k;
 }
 
 void free_colop(DevColOp& d) {

@@ -200,6 +200,7 @@ size_t pass_shared_bytes(int pass, int TI, int LP, int WPL, int LPW, int FPS) {
 }
 
 cudaError_t launch_pass(int pass, const PassArgs& a, int S, int WPL, cudaStream_t st) {
+  if (!a.opd.tab || !a.opf.tab) return cudaErrorInvalidValue;   // arguments without lane tables
   if (S == 3 && WPL == 1) return launch_pass_t<3, 1>(pass, a, st);
   if (S == 5 && WPL == 1) return launch_pass_t<5, 1>(pass, a, st);
   if (S == 5 && WPL == 2) return launch_pass_t<5, 2>(pass, a, st);

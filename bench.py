@@ -35,13 +35,13 @@ UNIT = "grid-point RK3 updates/s"
 B_ALG_STEP = 2504.0      # algorithmic bytes per unique grid point per RK3 step (pass model)
 B_ALG_STEP_FUSED = 2384.0   # the same with the owed filter along A fused into pass A
 # fields read + written per stored point by one launch of each pass (B' reads q for the c2 term at
-# two of the three stages; the filter along A owed by each stage is its own pass F_A where the
-# autotuner found that faster, else pass A filters first and moves 14 fields)
+# two of the three stages; A counts the primitives' 9 fields and its own 8, B 8; with the lane-scan
+# kernels pinned for pass A and the owed filter fused into it, A moves 14 fields)
 PASS_NAMES = ["A", "B", "C", "A'", "B'", "F", "diag", "F_A"]   # astr_pass_timings order
-PASS_FIELDS = {"A": 9, "B": 9, "C": 28, "A'": 15, "B'": 20 + 10 / 3, "F": 10, "F_A": 10}
+PASS_FIELDS = {"A": 17, "B": 8, "C": 28, "A'": 15, "B'": 20 + 10 / 3, "F": 10, "F_A": 10}
 PASS_PER_STEP = {"A": 3, "B": 3, "C": 3, "A'": 3, "B'": 3, "F": 3, "F_A": 3}
-# kernels of one filtered RK3 step in the timed region: 7 passes per stage (6 with filter-A fused
-# into pass A) and the diagnostics reduce
+# kernels of one filtered RK3 step in the timed region: 7 passes and the primitives per stage (6
+# passes with filter-A fused into the lane-scan pass A) and the diagnostics reduce
 
 
 def peaks():
@@ -302,7 +302,7 @@ def run_ours(args, ws, rank, local):
                        "l2": "inputs larger than L2 (5 x 1.1 GB state per box)", "graph": "one CUDA graph per step",
                        "launch_shapes": shapes},
             "roofline": roof, "step_roofline": step_roof, "cpu_baseline": cpu, "e2e": e2e,
-            "gpu_launches": (3 * (7 if split_fa else 6) + 1) * args.steps, "clocks": clk.summary(),
+            "gpu_launches": (3 * (8 if split_fa else 6) + 1) * args.steps, "clocks": clk.summary(),
             "adjoint": adjoint, "ensemble": ensemble, "checkpoint": checkpoint,
         }
         print(json.dumps(line), flush=True)

@@ -170,18 +170,20 @@ int astr_history(astr_state* st, double* rows, int maxrows, int* nrows);
 int astr_diagnostics(astr_state* st, double out[3]);
 /* Capture each RK3 step as one CUDA graph (default on). */
 int astr_state_use_graph(astr_state* st, int on);
-/* Apply the filter along y owed by each RK3 stage as its own pass (on) or fused into the first
- * gradient pass (off, the default); the autotuner times both at the first step and keeps the
- * faster unless this call (which turns autotuning off) or a pinned launch shape came first.
- * The two differ by rounding only (filterq, tgvsolver.F90:791-883). */
+/* Apply the filter along y owed by each RK3 stage as its own pass (on, the default) or fused into
+ * the first gradient pass (off; pass A then runs its lane-scan form). The call turns autotuning
+ * off. The two differ by rounding only (filterq, tgvsolver.F90:791-883). */
 int astr_state_split_filter(astr_state* st, int on);
 /* Per-pass autotuning of the launch shape (rows per lane, warps per line, lines per CTA) at the
- * first RK3 step of a state, on scratch copies of the live fields (default on above 100^3 nodes). */
+ * first RK3 step of a state, on scratch copies of the live fields (default on above 100^3 nodes),
+ * for the passes that run a lane-scan kernel: C and filter-C; the y and z passes run column solves
+ * whose shape follows from the box. */
 int astr_state_autotune(astr_state* st, int on);
 /* Launch shape of each pass A, B, C, A', B', filter-C, filter-A as (S, WPL, TI, LP, LPW, FPS):
- * 42 ints. */
+ * 42 ints. A pass that runs as a column solve reports its rows per chunk S, WPL 0 and its lines per
+ * CTA TI. */
 int astr_state_launch_shapes(astr_state* st, int shapes[42]);
-/* Pin pass `pass` (0..6 in the order above) to S rows per lane, WPL warps per line, TI lines per
+/* Pin pass `pass` (0..6 in the order above) to its lane-scan kernel with S rows per lane, WPL warps per line, TI lines per
  * CTA (a compiled layout whose 32*WPL*S rows cover the pass's line systems; TI a power of 2 with
  * (TI/LPW)*WPL*32 <= 512 threads, and TI/LPW <= 15 when WPL > 1) and
  * LPW lines per warp group (1; or a divisor of TI for the y/z passes A', B' and filter-A, whose

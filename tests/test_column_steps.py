@@ -1,0 +1,90 @@
+"""The y and z passes of the RK3 step as column solves (csrc/tgv_cols.cuh) against the oracle, on
+boxes whose y and z systems (N + 7 rows) sit at the edges where the rows per chunk (45, 90, 264,
+1056 rows), the lines per CTA (8 chunks) and the tile walk (x extent against 16 and 32 lines) change;
+with and without the filter, and with one pass at a time on its lane-scan kernel."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+# fields after a few steps: last-bit differences of the solves, scaled by each field's largest value
+TOL = 1e-12
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import astr_gpu_b200 as ag
+    return ag.Context(0)
+
+
+def _start(dims, seed):
+    """A smooth field with content along every axis, mach 0.3."""
+    rng = np.random.default_rng(seed)
+    x = [2 * np.pi * np.remainder(np.arange(n + 1), n) / n for n in dims]
+    X, Y, Z = np.meshgrid(*x, indexing="ij")
+    u = [np.sin(X) * np.cos(Y) * np.cos(Z), -np.cos(X) * np.sin(Y) * np.cos(Z), np.zeros_like(X)]
+    for _ in range(3):
+        k = rng.integers(1, 4, 3)
+        for c in range(3):
+            u[c] = u[c] + 0.1 * rng.standard_normal() * np.cos(k[0] * X + k[1] * Y + k[2] * Z + rng.uniform(0, 6))
+    p = 1.0 / (1.4 * 0.09) + 0.05 * np.cos(2 * X) * np.cos(Z)
+    rho = p * 1.4 * 0.09
+    q = np.stack([rho, rho * u[0], rho * u[1], rho * u[2], p / 0.4 + 0.5 * rho * (u[0]**2 + u[1]**2 + u[2]**2)], axis=-1)
+    return np.asfortranarray(q)
+
+
+def _oracle(dims, q0, dt, steps, filt):
+    o = oracle.TGVOracle(*dims, params=oracle.FlowParams(mach=0.3, reynolds=400.0, filter_on=filt))
+    o.set_q(q0)
+    o.set_dt(dt)
+    o.steps(steps)
+    return o.get_q()
+
+
+def _run(ctx, dims, q0, dt, steps, filt, pin=None):
+    import astr_gpu_b200 as ag
+    s = ag.TGVSolver(ctx, *dims, params=ag.FlowParams(mach=0.3, reynolds=400.0, filter_on=filt))
+    s.autotune(False)
+    if pin:
+        s.set_launch_shape(*pin)
+    s.set_q(q0)
+    s.rk3(dt, steps)
+    q = s.get_q()
+    s.close()
+    return q
+
+
+def _err(a, b):
+    return max(np.abs(a[..., m] - b[..., m]).max() / np.abs(b[..., m]).max() for m in range(5))
+
+
+@pytest.mark.parametrize("dims", [(16, 16, 16), (17, 20, 38), (31, 39, 19), (32, 83, 44), (33, 84, 16), (47, 16, 84),
+                                  (16, 257, 39), (20, 258, 38), (15 + 16, 60, 258), (16, 20, 300), (16, 1050, 16),
+                                  (600, 17, 18)])
+@pytest.mark.parametrize("filt", [True, False])
+def test_boxes(ctx, dims, filt):
+    q0 = _start(dims, sum(dims))
+    dt = 0.3 / ((1.5 + 1 / 0.3) * sum(n / (2 * np.pi) for n in dims))
+    assert _err(_run(ctx, dims, q0, dt, 2, filt), _oracle(dims, q0, dt, 2, filt)) <= TOL
+
+
+@pytest.mark.parametrize("name", ["A", "B", "A'", "B'", "F_A"])
+def test_one_pass_on_its_lane_scan_kernel(ctx, name):
+    """The two forms of a pass can be mixed: the primitives are stored by whichever gradient pass runs
+    as a column solve first."""
+    dims = (40, 56, 48)
+    q0 = _start(dims, 1)
+    pin = (name, 3, 1, 4)
+    assert _err(_run(ctx, dims, q0, 2e-3, 2, True, pin), _run(ctx, dims, q0, 2e-3, 2, True)) <= TOL
+
+
+def test_reported_shapes(ctx):
+    import astr_gpu_b200 as ag
+    s = ag.TGVSolver(ctx, 32, 128, 300)
+    sh = s.launch_shapes()
+    assert sh["A"] == (33, 0, 32, 0, 1, 1) and sh["B"] == (33, 0, 16, 0, 1, 1) and sh["C"][1] >= 1
+    s.set_launch_shape("B", 9, 2, 8)
+    assert s.launch_shapes()["B"][:3] == (9, 2, 8)
+    s.close()
