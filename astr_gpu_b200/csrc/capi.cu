@@ -59,7 +59,8 @@ struct astr_state {
   std::map<int, std::pair<DevOp, DevOp>> ops;   // lane tables per (direction, layout)
   PassCfg cfg[NCFG];                       // launch shape of every pass
   ColDir col[3];                           // column operators along y and z (x unused)
-  bool use_col[NCFG] = {true, true, false, true, true, false, true};   // passes run as column solves
+  RowOps rows;                             // and along x
+  bool use_col[NCFG] = {true, true, true, true, true, true, true};   // passes run as column solves
   bool autotune = true, tuned = false;
   bool pending = false;       // filter along DIR_A of the last stage not yet applied
   bool split_fa = true;       // that filter as its own pass (else fused into pass A)
@@ -263,7 +264,8 @@ std::pair<DevOp, DevOp>& get_ops(astr_state* st, int dir, int S, int WPL) {
 }
 
 // Number of pass-C CTAs, i.e. of partial sums the diagnostics reduce.
-int diag_parts(astr_state* st) {
+int diag_parts(astr_state* st, bool lane) {
+  if (!lane) return row_c_tiles(st->g, st->rows);
   const int o1 = (DIR_C == 0) ? 1 : 0, o2 = (DIR_C == 2) ? 1 : 2;
   const int ti = st->cfg[CFG_C].TI;
   return (int)(((st->g.N[o1] + 1 + ti - 1) / ti) * (int64_t)(st->g.N[o2] + 1));
@@ -294,6 +296,7 @@ PassArgs base_args(astr_state* st, int id, bool lane) {
   return a;
 }
 
+int diag_parts(astr_state* st) { return diag_parts(st, !st->use_col[CFG_C]); }
 PassArgs base_args(astr_state* st, int id) { return base_args(st, id, !st->use_col[id]); }
 
 // Optional per-pass event timing (astr_pass_timings); null in normal runs.
@@ -315,6 +318,8 @@ cudaError_t run_pass(astr_state* st, int id, PassArgs& a) {
   cudaStream_t sm = st->ctx->stream;
   cudaError_t e;
   if (!st->use_col[id]) e = launch_pass(pass, a, st->cfg[id].S, st->cfg[id].WPL, sm);
+  else if (id == CFG_C) e = launch_row_c(a, st->rows, sm);
+  else if (id == CFG_FC) e = launch_row_filter(a, st->rows, sm);
   else if (id == CFG_FA) e = launch_col_pass(0, a, nullptr, cd, sm);
   else if (id == CFG_VA) e = launch_col_pass(2, a, st->VF, cd, sm);
   else if (id == CFG_VB) e = launch_col_pass(a.mode == 0 ? 2 : 3, a, st->VF + 5 * st->g.fs, cd, sm);
@@ -791,8 +796,10 @@ int astr_state_create(astr_ctx* ctx, const astr_params* p, astr_state** out) {
     c.TI = pick_ti(pass_tiles(CFG_PASS[id]), N[d], L.WPL, L.S);
     c.LP = tile_pitch(N[d], c.TI, c.S);
   }
-  const cudaError_t ec = make_coldirs(st->hd, st->hf, st->col);
+  const cudaError_t ec = make_coldirs(st->hd, st->hf, st->col, st->rows);
   if (ec != cudaSuccess) { astr_state_destroy(st); return cuda_fail(ctx, ec, "column operators"); }
+  st->use_col[CFG_C] = st->rows.c.S != 0;
+  st->use_col[CFG_FC] = st->rows.f.S != 0;
   // a small box gains nothing from tuning
   st->autotune = (N[0] + 1) * (int64_t)(N[1] + 1) * (N[2] + 1) >= 100 * 100 * 100;
   // 33 fields: Q0(5) Q1(5) R(5) DA(4) DB(4) VF(10: the combined fluxes along A and along B)
@@ -974,7 +981,10 @@ int astr_state_launch_shapes(astr_state* st, int shapes[42]) {
   if (!st || !shapes) return ASTR_ERR_ARG;
   for (int id = 0; id < NCFG; ++id) {
     if (st->use_col[id]) {
-      const int col[6] = {st->col[CFG_DIR[id]].d.S, 0, col_lines(st->col[CFG_DIR[id]]), 0, 1, 1};
+      int col[6] = {st->col[CFG_DIR[id]].d.S, 0, 0, 0, 1, 1};
+      if (id == CFG_C) { col[0] = st->rows.c.S; col[2] = st->rows.c.NL; col[5] = 5; }
+      else if (id == CFG_FC) { col[0] = st->rows.f.S; col[2] = 8; }
+      else col[2] = col_lines(st->col[CFG_DIR[id]]);
       std::copy(col, col + 6, shapes + 6 * id);
       continue;
     }
@@ -1039,7 +1049,8 @@ int astr_rk3_step(astr_state* st, double dt, int nsteps) {
   if (!st || nsteps < 0 || !(dt > 0.0)) return ASTR_ERR_ARG;
   astr_ctx* ctx = st->ctx;
   if (hist_rows(st) + nsteps > st->hist_cap) return fail(ctx, ASTR_ERR_UNSUPPORTED, "history buffer full (65536 steps)");
-  if (st->autotune && !st->tuned && nsteps > 0) {
+  const bool lanes = !std::all_of(st->use_col, st->use_col + NCFG, [](bool c) { return c; });
+  if (st->autotune && !st->tuned && lanes && nsteps > 0) {
     drop_graphs(st);
     CK(autotune(st));
   }
@@ -1252,7 +1263,7 @@ int ens_build(astr_ensemble* e) {
             const int o1 = (dir == 0) ? 1 : 0, o2 = (dir == 2) ? 1 : 2;
             ctas += ((st->g.N[o1] + 1 + c.TI - 1) / c.TI) * (st->g.N[o2] + 1);
             L.smem = std::max(L.smem, pass_shared_bytes(L.pass, c.TI, c.LP, g.WPL));
-            if (id == CFG_C) hdiag[b].nparts = diag_parts(st);
+            if (id == CFG_C) hdiag[b].nparts = diag_parts(st, true);
           }
           L.nctas = ctas;
           if (id == CFG_FC && !e->boxes[0]->p.filter_on) continue;

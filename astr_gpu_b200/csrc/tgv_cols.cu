@@ -49,14 +49,18 @@ cudaError_t launch_dir(int pass, const ColArgs& a, const ColDir& d, int LW, int 
 
 int col_lines(const ColDir& d) { return lines_per_cta(d.d.op.nch); }
 
-cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out) {
-  ColSpec specs[4];
+cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out, RowOps& rows) {
+  ColSpec specs[6];
+  int n = 4;
+  rows.c = row_c_shape(hd[0].nsys());
+  if (rows.c.S) specs[n++] = ColSpec{&hd[0], rows.c.S, 0, &rows.d};
+  if (const int S = row_f_rows(hf[0].nsys())) specs[n++] = ColSpec{&hf[0], S, 0, &rows.f};
   for (int d = 1; d < 3; ++d) {
     const int S = col_rows_per_chunk(hf[d].nsys(), d);
     specs[2 * d - 2] = ColSpec{&hd[d], S, (hf[d].nsys() - hd[d].nsys()) / 2, &out[d].d};
     specs[2 * d - 1] = ColSpec{&hf[d], S, 0, &out[d].f};
   }
-  return make_colops(specs, 4);
+  return make_colops(specs, n);
 }
 
 void free_coldirs(ColDir* dirs) { free_colop(dirs[1].d); }

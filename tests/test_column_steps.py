@@ -1,6 +1,6 @@
-"""The y and z passes of the RK3 step as column solves (csrc/tgv_cols.cuh) against the oracle, on
-boxes whose y and z systems (N + 7 rows) sit at the edges where the rows per chunk (45, 90, 264,
-1056 rows), the lines per CTA (8 chunks) and the tile walk (x extent against 16 and 32 lines) change;
+"""The passes of the RK3 step as column solves (csrc/tgv_cols.cuh, tgv_rows.cuh) against the oracle, on
+boxes whose systems (N + 7 rows; N + 3 in pass C) sit at the edges where the rows per chunk, the lines
+per CTA and the tile walk (x extent against 16 and 32 lines, y extent against 2, 4 and 8) change;
 with and without the filter, and with one pass at a time on its lane-scan kernel."""
 import numpy as np
 import pytest
@@ -62,7 +62,12 @@ def _err(a, b):
 
 @pytest.mark.parametrize("dims", [(16, 16, 16), (17, 20, 38), (31, 39, 19), (32, 83, 44), (33, 84, 16), (47, 16, 84),
                                   (16, 257, 39), (20, 258, 38), (15 + 16, 60, 258), (16, 20, 300), (16, 1050, 16),
-                                  (600, 17, 18)])
+                                  (600, 17, 18),
+                                  # the x passes: rows per chunk, lines per CTA, the widest boxes
+                                  (38, 16, 17), (39, 17, 16), (42, 23, 17), (43, 24, 16), (99, 17, 16), (100, 18, 16),
+                                  (169, 16, 16), (170, 25, 16), (201, 16, 17), (202, 17, 16), (297, 19, 16), (298, 16, 16),
+                                  (622, 17, 16), (623, 16, 17), (822, 16, 16), (823, 17, 16), (1049, 16, 16),
+                                  (1050, 16, 17)])
 @pytest.mark.parametrize("filt", [True, False])
 def test_boxes(ctx, dims, filt):
     q0 = _start(dims, sum(dims))
@@ -70,7 +75,7 @@ def test_boxes(ctx, dims, filt):
     assert _err(_run(ctx, dims, q0, dt, 2, filt), _oracle(dims, q0, dt, 2, filt)) <= TOL
 
 
-@pytest.mark.parametrize("name", ["A", "B", "A'", "B'", "F_A"])
+@pytest.mark.parametrize("name", ["A", "B", "C", "A'", "B'", "F_C", "F_A"])
 def test_one_pass_on_its_lane_scan_kernel(ctx, name):
     """The two forms of a pass can be mixed: the primitives are stored by whichever gradient pass runs
     as a column solve first."""
@@ -84,7 +89,7 @@ def test_reported_shapes(ctx):
     import astr_gpu_b200 as ag
     s = ag.TGVSolver(ctx, 32, 128, 300)
     sh = s.launch_shapes()
-    assert sh["A"] == (33, 0, 32, 0, 1, 1) and sh["B"] == (33, 0, 16, 0, 1, 1) and sh["C"][1] >= 1
+    assert sh["A"] == (33, 0, 32, 0, 1, 1) and sh["B"] == (33, 0, 16, 0, 1, 1) and sh["C"] == (9, 0, 8, 0, 1, 5) and sh["F_C"] == (9, 0, 8, 0, 1, 1)
     s.set_launch_shape("B", 9, 2, 8)
     assert s.launch_shapes()["B"][:3] == (9, 2, 8)
     s.close()
