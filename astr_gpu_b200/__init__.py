@@ -156,8 +156,8 @@ def _apply(ctx, scheme, f, direction, lbound, out_lbound, out_shape, scale, kind
         assert f.is_cuda and f.dtype == torch.float64
         # Fortran order <=> the tensor's strides are column-major
         fp = f
-        out = torch.empty(tuple(oshape) + ((nf,) if f.ndim == 4 else ()), dtype=torch.float64, device=f.device)
-        out = out.permute(*reversed(range(out.ndim))).contiguous().permute(*reversed(range(out.ndim)))
+        dims = tuple(oshape) + ((nf,) if f.ndim == 4 else ())
+        out = torch.empty(dims[::-1], dtype=torch.float64, device=f.device).permute(*reversed(range(len(dims))))
         assert fp.stride(0) == 1 and out.stride(0) == 1, "device arrays must be Fortran-ordered"
         torch.cuda.current_stream(f.device).synchronize()
         fptr, optr, where = fp.data_ptr(), out.data_ptr(), ASTR_DEVICE
