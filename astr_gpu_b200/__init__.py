@@ -525,8 +525,8 @@ class FullSolver:
 
 class Ensemble:
     """Independent periodic boxes (``TGVSolver`` objects of one context, sizes may differ)
-    advanced together: each pass of an RK3 stage is one launch over every box sharing a solve
-    layout, and each step is one CUDA graph. Per-box results equal ``TGVSolver.rk3``."""
+    advanced together: each step is one CUDA graph with every box's passes on branches of their
+    own. Per-box results equal ``TGVSolver.rk3``."""
 
     def __init__(self, ctx: Context, boxes: list[TGVSolver]):
         self.ctx = ctx

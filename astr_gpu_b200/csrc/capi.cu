@@ -8,7 +8,6 @@
 #include <map>
 #include <new>
 #include <string>
-#include <array>
 #include <vector>
 
 #include "../../include/astr_b200.h"
@@ -67,35 +66,20 @@ struct astr_state {
   int nstep = 0;
   double time = 0.0;
   std::vector<double> row_key;  // (nstep, time) per history row
+  cudaStream_t run = nullptr;         // stream of the passes while an ensemble captures (else the context's)
+  const double* pdt = nullptr;        // the time step on the device, likewise
   bool use_graph = true;
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   double gdt[2] = {0.0, 0.0};
 };
 
-// One launch of the batched step: a pass over the boxes of one solve layout, or the batched
-// diagnostics reduce (pass == 0).
-struct EnsLaunch {
-  int pass = 0, dir = 0, S = 0, WPL = 0, nbox = 0, nctas = 0, threads = 0;
-  size_t smem = 0, args_off = 0, cum_off = 0;
-};
-
 struct astr_ensemble {
   astr_ctx* ctx = nullptr;
   std::vector<astr_state*> boxes;
-  struct Group {
-    int S = 0, WPL = 0;
-    std::vector<int> members;
-    int TI[NCFG] = {0};
-  };
-  std::vector<Group> groups;
-  PassArgs* dargs = nullptr;
-  int* dcum = nullptr;
-  DiagArgs* ddiag = nullptr;
-  std::vector<EnsLaunch> plan[2];   // per variant: filter along A owed at the start of the step or not
   std::vector<double> dt;
-  cudaGraphExec_t gexec[2] = {nullptr, nullptr};
+  double* ddt = nullptr;            // the boxes' time steps on the device
+  cudaGraphExec_t gexec[2] = {nullptr, nullptr};   // filter along A owed at the start of the step or not
   bool pending = false;
-  bool tuned = false;
 };
 
 namespace {
@@ -243,7 +227,7 @@ int scheme_tables(astr_ctx* ctx, astr_scheme* s, astr_scheme** out) {
   const int nsys = s->h.nsys();
   if (col_rows_per_chunk(nsys, 0) == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
   const ColSpec specs[2] = {{&s->h, col_rows_per_chunk(nsys, 0), 0, &s->d[0]}, {&s->h, col_rows_per_chunk(nsys, 1), 0, &s->d[1]}};
-  const cudaError_t e = make_colops(specs, 2);
+  const cudaError_t e = make_colops(specs, 2, ctx->stream);
   if (e != cudaSuccess) {
     free_colop(s->d[0]);
     delete s;
@@ -264,22 +248,21 @@ std::pair<DevOp, DevOp>& get_ops(astr_state* st, int dir, int S, int WPL) {
 }
 
 // Number of pass-C CTAs, i.e. of partial sums the diagnostics reduce.
-int diag_parts(astr_state* st, bool lane) {
-  if (!lane) return row_c_tiles(st->g, st->rows);
+int diag_parts(astr_state* st) {
+  if (st->use_col[CFG_C]) return row_c_tiles(st->g, st->rows);
   const int o1 = (DIR_C == 0) ? 1 : 0, o2 = (DIR_C == 2) ? 1 : 2;
   const int ti = st->cfg[CFG_C].TI;
   return (int)(((st->g.N[o1] + 1 + ti - 1) / ti) * (int64_t)(st->g.N[o2] + 1));
 }
 
-// Arguments of pass `id`; lane: with the tables of its lane-scan kernel (which the batched ensemble
-// passes always run).
-PassArgs base_args(astr_state* st, int id, bool lane) {
+// Arguments of pass `id`, with the tables of its lane-scan kernel where it runs that.
+PassArgs base_args(astr_state* st, int id) {
   const PassCfg& pc = st->cfg[id];
   const int dir = CFG_DIR[id];
   PassArgs a{};
   a.g = st->g;
   a.th = st->th;
-  if (lane) {
+  if (!st->use_col[id]) {
     auto& o = get_ops(st, dir, pc.S, pc.WPL);
     a.opd = o.first.op;
     a.opf = o.second.op;
@@ -295,9 +278,6 @@ PassArgs base_args(astr_state* st, int id, bool lane) {
   a.err = st->err;
   return a;
 }
-
-int diag_parts(astr_state* st) { return diag_parts(st, !st->use_col[CFG_C]); }
-PassArgs base_args(astr_state* st, int id) { return base_args(st, id, !st->use_col[id]); }
 
 // Optional per-pass event timing (astr_pass_timings); null in normal runs.
 struct PassTimer {
@@ -315,7 +295,7 @@ cudaError_t run_pass(astr_state* st, int id, PassArgs& a) {
     cudaEventRecord(e0, st->ctx->stream);
   }
   const ColDir& cd = st->col[a.dir];
-  cudaStream_t sm = st->ctx->stream;
+  cudaStream_t sm = st->run ? st->run : st->ctx->stream;
   cudaError_t e;
   if (!st->use_col[id]) e = launch_pass(pass, a, st->cfg[id].S, st->cfg[id].WPL, sm);
   else if (id == CFG_C) e = launch_row_c(a, st->rows, sm);
@@ -398,7 +378,7 @@ cudaError_t run_step(astr_state* st, double dt, bool pending_at_start) {
       const double norm = (double)st->p.im * (double)st->p.jm * (double)st->p.km;
       cudaEvent_t e0 = nullptr, e1 = nullptr;
       if (g_timer) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, st->ctx->stream); }
-      if ((e = launch_diag_reduce(st->partials, diag_parts(st), st->hist, st->counter, norm, st->ctx->stream)) != cudaSuccess)
+      if ((e = launch_diag_reduce(st->partials, diag_parts(st), st->hist, st->counter, norm, st->run ? st->run : st->ctx->stream)) != cudaSuccess)
         return e;
       if (g_timer) {
         cudaEventRecord(e1, st->ctx->stream);
@@ -411,7 +391,7 @@ cudaError_t run_step(astr_state* st, double dt, bool pending_at_start) {
     a = base_args(st, CFG_VB);
     a.q = qin; a.qsave = st->Q0; a.qout = qout;
     a.mode = 1; a.do_filter = filt;
-    a.c1 = rk[s][0]; a.c2 = rk[s][1]; a.c3 = rk[s][2]; a.dt = dt;
+    a.c1 = rk[s][0]; a.c2 = rk[s][1]; a.c3 = rk[s][2]; a.dt = dt; a.pdt = st->pdt;
     if ((e = run_pass(st, CFG_VB, a)) != cudaSuccess) return e;
     if (filt) {
       a = base_args(st, CFG_FC);
@@ -594,6 +574,12 @@ cudaError_t autotune(astr_state* st) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
   st->tuned = true;
   return e;
+}
+
+// Whether a state's first step still times the launch shapes of its lane-scan passes.
+bool wants_tuning(const astr_state* st) {
+  const bool lanes = !std::all_of(st->use_col, st->use_col + NCFG, [](bool c) { return c; });
+  return st->autotune && !st->tuned && lanes;
 }
 
 void drop_graphs(astr_state* st) {
@@ -796,7 +782,7 @@ int astr_state_create(astr_ctx* ctx, const astr_params* p, astr_state** out) {
     c.TI = pick_ti(pass_tiles(CFG_PASS[id]), N[d], L.WPL, L.S);
     c.LP = tile_pitch(N[d], c.TI, c.S);
   }
-  const cudaError_t ec = make_coldirs(st->hd, st->hf, st->col, st->rows);
+  const cudaError_t ec = make_coldirs(st->hd, st->hf, st->col, st->rows, ctx->stream);
   if (ec != cudaSuccess) { astr_state_destroy(st); return cuda_fail(ctx, ec, "column operators"); }
   st->use_col[CFG_C] = st->rows.c.S != 0;
   st->use_col[CFG_FC] = st->rows.f.S != 0;
@@ -1049,8 +1035,7 @@ int astr_rk3_step(astr_state* st, double dt, int nsteps) {
   if (!st || nsteps < 0 || !(dt > 0.0)) return ASTR_ERR_ARG;
   astr_ctx* ctx = st->ctx;
   if (hist_rows(st) + nsteps > st->hist_cap) return fail(ctx, ASTR_ERR_UNSUPPORTED, "history buffer full (65536 steps)");
-  const bool lanes = !std::all_of(st->use_col, st->use_col + NCFG, [](bool c) { return c; });
-  if (st->autotune && !st->tuned && lanes && nsteps > 0) {
+  if (wants_tuning(st) && nsteps > 0) {
     drop_graphs(st);
     CK(autotune(st));
   }
@@ -1187,204 +1172,67 @@ int astr_diagnostics(astr_state* st, double out[3]) {
 }  // extern "C"
 
 // ====================================================================== batched ensemble
-// Many independent periodic boxes of uneven sizes advanced together: boxes are grouped by the
-// solve layout their size selects, and every pass of a stage is one launch per group whose
-// CTAs walk the concatenated tile grids of the group's boxes (launch_pass_batch); the stage's
-// diagnostics reduce is one launch for all boxes. Each ensemble step is one CUDA graph.
+// Many independent periodic boxes of uneven sizes advanced together: an ensemble step is one CUDA
+// graph in which every box's step is a chain of its own passes, on up to ENS_BRANCHES parallel
+// branches, so the launches of small boxes run beside those of the others and no box waits for
+// another between passes. The time steps are read from device memory: changing them keeps the graph.
 namespace {
+
+constexpr int ENS_BRANCHES = 32;   // kernels of this many boxes in flight; more boxes share branches
 
 void ens_drop_graphs(astr_ensemble* e) {
   for (auto& g : e->gexec)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
 
-void ens_free_plan(astr_ensemble* e) {
-  if (e->dargs) cudaFree(e->dargs);
-  if (e->dcum) cudaFree(e->dcum);
-  if (e->ddiag) cudaFree(e->ddiag);
-  e->dargs = nullptr; e->dcum = nullptr; e->ddiag = nullptr;
+int64_t box_nodes(const astr_state* st) {
+  return (int64_t)(st->g.N[0] + 1) * (st->g.N[1] + 1) * (st->g.N[2] + 1);
 }
 
-// Build the launch plans of both variants for the current dt and upload their arguments.
-int ens_build(astr_ensemble* e) {
+// The step of every box as one graph: boxes by decreasing size, each to the branch with the least work.
+int ens_capture(astr_ensemble* e, int variant) {
   astr_ctx* ctx = e->ctx;
-  static const double rk[3][3] = {{1.0, 0.0, 1.0}, {0.75, 0.25, 0.25}, {1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0}};
-  std::vector<PassArgs> hargs;
-  std::vector<int> hcum;
-  std::vector<DiagArgs> hdiag;
-  for (astr_state* st : e->boxes) {
-    DiagArgs d;
-    d.partials = st->partials; d.nparts = 0; d.hist = st->hist; d.counter = st->counter;
-    d.norm = (double)st->p.im * (double)st->p.jm * (double)st->p.km;
-    hdiag.push_back(d);
-  }
-  const int slots[6] = {CFG_A, CFG_B, CFG_C, CFG_VA, CFG_VB, CFG_FC};
-  // base_args reads a box's launch configuration: lend it the group's for the build only.
-  std::vector<std::array<PassCfg, NCFG>> saved(e->boxes.size());
-  for (size_t b = 0; b < e->boxes.size(); ++b)
-    for (int id = 0; id < NCFG; ++id) saved[b][id] = e->boxes[b]->cfg[id];
-  for (int variant = 0; variant < 2; ++variant) {
-    e->plan[variant].clear();
-    for (int s = 0; s < 3; ++s) {
-      for (int si = 0; si < 6; ++si) {
-        const int id = slots[si];
-        for (auto& g : e->groups) {
-          EnsLaunch L;
-          L.pass = CFG_PASS[id]; L.dir = CFG_DIR[id]; L.S = g.S; L.WPL = g.WPL;
-          L.nbox = (int)g.members.size();
-          L.threads = g.TI[id] * g.WPL * 32;
-          L.args_off = hargs.size();
-          L.cum_off = hcum.size();
-          int ctas = 0;
-          for (int b : g.members) {
-            astr_state* st = e->boxes[b];
-            const int dir = CFG_DIR[id];
-            PassCfg c;
-            c.S = g.S; c.WPL = g.WPL; c.TI = g.TI[id]; c.LP = tile_pitch(st->g.N[dir], c.TI, g.S);
-            st->cfg[id] = c;
-            PassArgs a = base_args(st, id, true);
-            double* qin = (s == 0) ? st->Q0 : st->Q1;
-            double* qout = (s == 2) ? st->Q0 : st->Q1;
-            const int filt = st->p.filter_on;
-            switch (id) {
-              case CFG_A: a.q = qin; a.D = st->DA; a.do_filter = filt && (s > 0 || variant == 1); break;
-              case CFG_B: a.q = qin; a.D = st->DB; break;
-              case CFG_C: a.q = qin; a.DA = st->DA; a.DB = st->DB; a.partials = (s == 0) ? st->partials : nullptr; break;
-              case CFG_VA: a.q = qin; break;
-              case CFG_VB:
-                a.q = qin; a.qsave = st->Q0; a.qout = qout; a.mode = 1; a.do_filter = filt;
-                a.c1 = rk[s][0]; a.c2 = rk[s][1]; a.c3 = rk[s][2]; a.dt = e->dt[b];
-                break;
-              case CFG_FC: a.q = qout; break;
-              default: break;
-            }
-            hargs.push_back(a);
-            hcum.push_back(ctas);
-            const int o1 = (dir == 0) ? 1 : 0, o2 = (dir == 2) ? 1 : 2;
-            ctas += ((st->g.N[o1] + 1 + c.TI - 1) / c.TI) * (st->g.N[o2] + 1);
-            L.smem = std::max(L.smem, pass_shared_bytes(L.pass, c.TI, c.LP, g.WPL));
-            if (id == CFG_C) hdiag[b].nparts = diag_parts(st, true);
-          }
-          L.nctas = ctas;
-          if (id == CFG_FC && !e->boxes[0]->p.filter_on) continue;
-          e->plan[variant].push_back(L);
-        }
-        if (s == 0 && id == CFG_C) {   // the stage-1 diagnostics of every box
-          EnsLaunch L;
-          L.pass = 0; L.nbox = (int)e->boxes.size();
-          e->plan[variant].push_back(L);
-        }
-      }
+  const int nbox = (int)e->boxes.size(), nbr = std::min(nbox, ENS_BRANCHES);
+  std::vector<int> order(nbox);
+  for (int b = 0; b < nbox; ++b) order[b] = b;
+  std::sort(order.begin(), order.end(), [&](int x, int y) { return box_nodes(e->boxes[x]) > box_nodes(e->boxes[y]); });
+  std::vector<int64_t> load(nbr, 0);
+  std::vector<cudaStream_t> strm(nbr, nullptr);
+  std::vector<cudaEvent_t> ev(nbr + 1, nullptr);
+  cudaError_t err = cudaSuccess;
+  for (auto& x : strm)
+    if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking);
+  for (auto& x : ev)
+    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+  cudaGraph_t graph = nullptr;
+  if (err == cudaSuccess) err = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
+  if (err == cudaSuccess) {
+    err = cudaEventRecord(ev[nbr], ctx->stream);
+    for (int k = 0; k < nbr && err == cudaSuccess; ++k) err = cudaStreamWaitEvent(strm[k], ev[nbr], 0);
+    for (int i = 0; i < nbox && err == cudaSuccess; ++i) {
+      const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      astr_state* st = e->boxes[order[i]];
+      load[k] += box_nodes(st);
+      st->run = strm[k];
+      st->pdt = e->ddt + order[i];
+      err = run_step(st, e->dt[order[i]], variant == 1);
+      st->run = nullptr;
+      st->pdt = nullptr;
     }
-  }
-  for (size_t b = 0; b < e->boxes.size(); ++b)
-    for (int id = 0; id < NCFG; ++id) e->boxes[b]->cfg[id] = saved[b][id];
-  ens_free_plan(e);
-  CK(cudaMalloc(&e->dargs, hargs.size() * sizeof(PassArgs)));
-  CK(cudaMalloc(&e->dcum, hcum.size() * sizeof(int)));
-  CK(cudaMalloc(&e->ddiag, hdiag.size() * sizeof(DiagArgs)));
-  CK(cudaMemcpy(e->dargs, hargs.data(), hargs.size() * sizeof(PassArgs), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(e->dcum, hcum.data(), hcum.size() * sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(e->ddiag, hdiag.data(), hdiag.size() * sizeof(DiagArgs), cudaMemcpyHostToDevice));
-  return ASTR_OK;
-}
-
-cudaError_t ens_run(astr_ensemble* e, int variant) {
-  cudaStream_t sm = e->ctx->stream;
-  for (const EnsLaunch& L : e->plan[variant]) {
-    cudaError_t err;
-    if (L.pass == 0) err = launch_diag_reduce_batch(e->ddiag, L.nbox, sm);
-    else err = launch_pass_batch(L.pass, L.dir, L.S, L.WPL, e->dargs + L.args_off, e->dcum + L.cum_off, L.nbox, L.nctas,
-                                 L.threads, L.smem, sm);
-    if (err != cudaSuccess) return err;
-  }
-  return cudaSuccess;
-}
-
-// Lines per CTA of each pass of each group: start from the largest power of two (<= 512
-// threads) whose tiles fit in ~110 KB for every box of the group; with `timed`, also time the
-// batched launch of each pass at that width, half and a quarter of it on scratch copies of the
-// boxes' states (Q1) and keep the fastest.
-int ens_tune(astr_ensemble* e, bool timed) {
-  astr_ctx* ctx = e->ctx;
-  for (auto& g : e->groups) {
-    for (int id = 0; id < NCFG; ++id) {
-      int ti = 16;
-      for (int b : g.members) ti = std::min(ti, pick_ti(pass_tiles(CFG_PASS[id]), e->boxes[b]->g.N[CFG_DIR[id]], g.WPL, g.S));
-      g.TI[id] = std::max(ti, 1);
+    for (int k = 0; k < nbr && err == cudaSuccess; ++k) {
+      err = cudaEventRecord(ev[k], strm[k]);
+      if (err == cudaSuccess) err = cudaStreamWaitEvent(ctx->stream, ev[k], 0);
     }
+    const cudaError_t end = cudaStreamEndCapture(ctx->stream, &graph);
+    if (err == cudaSuccess) err = end;
   }
-  if (!timed) return ASTR_OK;
-  cudaStream_t sm = ctx->stream;
-  for (astr_state* st : e->boxes)
-    CK(cudaMemcpyAsync(st->Q1, st->Q0, 5 * (size_t)st->g.fs * sizeof(double), cudaMemcpyDeviceToDevice, sm));
-  PassArgs* dargs = nullptr;
-  int* dcum = nullptr;
-  CK(cudaMalloc(&dargs, e->boxes.size() * sizeof(PassArgs)));
-  CK(cudaMalloc(&dcum, e->boxes.size() * sizeof(int)));
-  cudaEvent_t t0, t1;
-  cudaEventCreate(&t0);
-  cudaEventCreate(&t1);
-  const int ids[6] = {CFG_A, CFG_B, CFG_C, CFG_VA, CFG_VB, CFG_FC};
-  for (auto& g : e->groups) {
-    for (int id : ids) {
-      const int ti0 = g.TI[id];
-      float best = 1e30f;
-      int best_ti = ti0;
-      for (int ti : {ti0, ti0 / 2, ti0 / 4}) {
-        if (ti < 1) continue;
-        std::vector<PassArgs> ha;
-        std::vector<int> hc;
-        int ctas = 0;
-        size_t smem = 0;
-        for (int b : g.members) {
-          astr_state* st = e->boxes[b];
-          const int dir = CFG_DIR[id];
-          const PassCfg saved = st->cfg[id];
-          PassCfg c;
-          c.S = g.S; c.WPL = g.WPL; c.TI = ti; c.LP = tile_pitch(st->g.N[dir], ti, g.S);
-          st->cfg[id] = c;
-          PassArgs a = base_args(st, id, true);
-          st->cfg[id] = saved;
-          a.q = st->Q1; a.D = st->DA; a.DA = st->DA; a.DB = st->DB; a.partials = nullptr;
-          // stage 2-3 form of the update: q (scratch) and qsave (live state, only read) distinct
-          a.qsave = st->Q0; a.qout = st->Q1; a.mode = 1; a.do_filter = st->p.filter_on;
-          a.c1 = 0.5; a.c2 = 0.5; a.c3 = 0.0; a.dt = 0.0;
-          ha.push_back(a);
-          hc.push_back(ctas);
-          const int o1 = (dir == 0) ? 1 : 0, o2 = (dir == 2) ? 1 : 2;
-          ctas += ((st->g.N[o1] + 1 + ti - 1) / ti) * (st->g.N[o2] + 1);
-          smem = std::max(smem, pass_shared_bytes(CFG_PASS[id], ti, c.LP, g.WPL));
-        }
-        CK(cudaMemcpyAsync(dargs, ha.data(), ha.size() * sizeof(PassArgs), cudaMemcpyHostToDevice, sm));
-        CK(cudaMemcpyAsync(dcum, hc.data(), hc.size() * sizeof(int), cudaMemcpyHostToDevice, sm));
-        const int threads = ti * g.WPL * 32;
-        float ms = 1e30f;
-        cudaError_t err = launch_pass_batch(CFG_PASS[id], CFG_DIR[id], g.S, g.WPL, dargs, dcum, (int)ha.size(), ctas,
-                                            threads, smem, sm);
-        if (err == cudaSuccess) {
-          cudaEventRecord(t0, sm);
-          for (int r = 0; r < 2 && err == cudaSuccess; ++r)
-            err = launch_pass_batch(CFG_PASS[id], CFG_DIR[id], g.S, g.WPL, dargs, dcum, (int)ha.size(), ctas, threads,
-                                    smem, sm);
-          cudaEventRecord(t1, sm);
-          cudaEventSynchronize(t1);
-          cudaEventElapsedTime(&ms, t0, t1);
-        }
-        if (err != cudaSuccess) { cudaGetLastError(); ms = 1e30f; }   // a width the device cannot launch
-        if (ms < best) { best = ms; best_ti = ti; }
-      }
-      g.TI[id] = best_ti;
-    }
-  }
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
-  cudaFree(dargs);
-  cudaFree(dcum);
-  for (astr_state* st : e->boxes) CK(cudaMemsetAsync(st->err, 0, sizeof(int), sm));
-  CK(cudaStreamSynchronize(sm));
-  e->tuned = true;
-  return ASTR_OK;
+  if (err == cudaSuccess) err = cudaGraphInstantiate(&e->gexec[variant], graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  for (auto x : ev)
+    if (x) cudaEventDestroy(x);
+  for (auto x : strm)
+    if (x) cudaStreamDestroy(x);
+  return err == cudaSuccess ? ASTR_OK : cuda_fail(ctx, err, "ensemble step capture");
 }
 
 }  // namespace
@@ -1401,22 +1249,10 @@ int astr_ensemble_create(astr_ctx* ctx, astr_state* const* boxes, int nbox, astr
     if (boxes[b]->p.filter_on != boxes[0]->p.filter_on) { delete e; return fail(ctx, ASTR_ERR_ARG, "mixed filter_on"); }
     e->boxes.push_back(boxes[b]);
   }
-  for (int b = 0; b < nbox; ++b) {
-    astr_state* st = boxes[b];
-    int mx = 0;
-    for (int d = 0; d < 3; ++d) mx = std::max(mx, st->hf[d].nsys());
-    const Layout L = pick_layout(mx);
-    bool found = false;
-    for (auto& g : e->groups)
-      if (g.S == L.S && g.WPL == L.WPL) { g.members.push_back(b); found = true; }
-    if (!found) {
-      astr_ensemble::Group g;
-      g.S = L.S; g.WPL = L.WPL;
-      g.members.push_back(b);
-      e->groups.push_back(g);
-    }
+  if (cudaMalloc(&e->ddt, (size_t)nbox * sizeof(double)) != cudaSuccess) {
+    delete e;
+    return fail(ctx, ASTR_ERR_NOMEM, "ensemble allocation");
   }
-  ens_tune(e, false);
   *out = e;
   return ASTR_OK;
 }
@@ -1425,7 +1261,7 @@ int astr_ensemble_destroy(astr_ensemble* e) {
   const DeviceGuard dg_(e ? e->ctx->device : -1);
   if (!e) return ASTR_ERR_ARG;
   ens_drop_graphs(e);
-  ens_free_plan(e);
+  cudaFree(e->ddt);
   delete e;
   return ASTR_OK;
 }
@@ -1448,16 +1284,14 @@ int astr_ensemble_step(astr_ensemble* e, const double* dt, int nsteps) {
   if (!all_pending)
     for (int b = 0; b < nbox; ++b) CK(finalize_filter(e->boxes[b]));
   e->pending = all_pending;
-  if (!e->tuned && nsteps > 0) {
-    int rc = ens_tune(e, true);
-    if (rc) return rc;
-    changed = true;
-  }
   if (changed) {
     e->dt.assign(dt, dt + nbox);
-    ens_drop_graphs(e);
-    int rc = ens_build(e);
-    if (rc) return rc;
+    CK(cudaMemcpyAsync(e->ddt, dt, (size_t)nbox * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  }
+  for (int b = 0; b < nbox && nsteps > 0; ++b) {
+    astr_state* st = e->boxes[b];
+    if (wants_tuning(st)) CK(autotune(st));
+    if (changed && !st->use_col[CFG_VB]) ens_drop_graphs(e);   // its update takes the time step by value
   }
   for (int s = 0; s < nsteps; ++s) {
     const int variant = e->pending ? 1 : 0;
@@ -1467,14 +1301,8 @@ int astr_ensemble_step(astr_ensemble* e, const double* dt, int nsteps) {
       st->row_key.push_back(st->time);
     }
     if (!e->gexec[variant]) {
-      cudaGraph_t graph;
-      CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
-      cudaError_t err = ens_run(e, variant);
-      cudaError_t err2 = cudaStreamEndCapture(ctx->stream, &graph);
-      if (err != cudaSuccess) return cuda_fail(ctx, err, "ensemble step capture");
-      if (err2 != cudaSuccess) return cuda_fail(ctx, err2, "cudaStreamEndCapture");
-      CK(cudaGraphInstantiate(&e->gexec[variant], graph, 0));
-      cudaGraphDestroy(graph);
+      const int rc = ens_capture(e, variant);
+      if (rc) return rc;
     }
     CK(cudaGraphLaunch(e->gexec[variant], ctx->stream));
     e->pending = e->boxes[0]->p.filter_on != 0;

@@ -1063,7 +1063,7 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
       return ASTR_ERR_UNSUPPORTED;
     }
   }
-  if (make_colops(specs.data(), (int)specs.size()) != cudaSuccess) {
+  if (make_colops(specs.data(), (int)specs.size(), astr_ctx_stream(ctx)) != cudaSuccess) {
     astr_full_destroy(fs);
     astr_ctx_set_error(ctx, "scheme tables");
     return ASTR_ERR_CUDA;

@@ -67,7 +67,7 @@ struct ColSpec {
   int S, pad;      // rows per chunk, identity rows around the system
   DevColOp* out;
 };
-cudaError_t make_colops(const ColSpec* specs, int n);   // one allocation, freed with the first
+cudaError_t make_colops(const ColSpec* specs, int n, cudaStream_t st);   // one allocation, freed with the first
 void free_colop(DevColOp& d);
 // Right-hand side weights for an output scaled by `scale`.
 ColWeights col_weights(const DevColOp& d, double scale);

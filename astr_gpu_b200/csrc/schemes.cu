@@ -381,7 +381,7 @@ static cudaError_t fill_colop(const HostOp& h, int S, int pad, DevColOp& out, st
 }
 
 // Column operators share one device table, owned by the first of them.
-cudaError_t make_colops(const ColSpec* specs, int n) {
+cudaError_t make_colops(const ColSpec* specs, int n, cudaStream_t st) {
   std::vector<double> all;
   std::vector<size_t> at(n);
   for (int i = 0; i < n; ++i) {
@@ -396,7 +396,9 @@ cudaError_t make_colops(const ColSpec* specs, int n) {
   DevColOp& own = *specs[0].out;
   cudaError_t e = cudaMalloc(&own.dtab, all.size() * sizeof(double));
   if (e != cudaSuccess) return e;
-  e = cudaMemcpy(own.dtab, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice);
+  // on the context's stream: a copy on the legacy stream would wait for the caller's work there
+  e = cudaMemcpyAsync(own.dtab, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   for (int i = 0; i < n; ++i) specs[i].out->op.tab = own.dtab + at[i];
   return e;
 }

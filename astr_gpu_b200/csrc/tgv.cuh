@@ -45,6 +45,7 @@ struct PassArgs {
   int do_filter;
   int mode;                 // pass B': 0 = only R += visc_B, 1 = RK update (+ filter)
   double c1, c2, c3, dt;    // SSP-RK3 stage coefficients (mainloop.F90:350-360)
+  const double* pdt;        // column passes: dt read from the device when not null
   double* partials;         // pass C at the first stage: per-CTA (tke, enstrophy, dissipation)
   double* DC;               // pass C, optional: its 4 gradients along C are also stored here
   int* err;                 // device error word: bit 0 = non-finite or non-positive density,
@@ -53,24 +54,10 @@ struct PassArgs {
 
 cudaError_t launch_pass(int pass, const PassArgs& a, int S, int WPL, cudaStream_t st);
 int pass_tiles(int pass);
-// One launch of a pass over nbox boxes of one solve layout: dargs[k] are box k's arguments
-// (device memory), dcum[k] its first CTA, nctas the total.
-cudaError_t launch_pass_batch(int pass, int dir, int S, int WPL, const PassArgs* dargs, const int* dcum, int nbox,
-                              int nctas, int threads, size_t smem, cudaStream_t st);
 size_t pass_shared_bytes(int pass, int TI, int LP, int WPL, int LPW = 1, int FPS = 5);
 // Field tiles of a pass's shared memory for a launch shape (LPW lines per warp group, FPS fields
 // per step of the streaming passes).
 int shape_tiles(int pass, int LPW, int FPS);
-
-// Batched diagnostics reduce: one CTA per box.
-struct DiagArgs {
-  const double* partials;
-  int nparts;
-  double* hist;
-  int* counter;
-  double norm;
-};
-cudaError_t launch_diag_reduce_batch(const DiagArgs* dargs, int nbox, cudaStream_t st);
 
 // Final ordered reduction of the pass-C partial sums into the history buffer.
 cudaError_t launch_diag_reduce(const double* partials, int nparts, double* hist, int* counter, double norm,

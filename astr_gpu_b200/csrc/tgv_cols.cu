@@ -49,7 +49,7 @@ cudaError_t launch_dir(int pass, const ColArgs& a, const ColDir& d, int LW, int 
 
 int col_lines(const ColDir& d) { return lines_per_cta(d.d.op.nch); }
 
-cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out, RowOps& rows) {
+cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out, RowOps& rows, cudaStream_t st) {
   ColSpec specs[6];
   int n = 4;
   rows.c = row_c_shape(hd[0].nsys());
@@ -60,7 +60,7 @@ cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out, RowOps
     specs[2 * d - 2] = ColSpec{&hd[d], S, (hf[d].nsys() - hd[d].nsys()) / 2, &out[d].d};
     specs[2 * d - 1] = ColSpec{&hf[d], S, 0, &out[d].f};
   }
-  return make_colops(specs, n);
+  return make_colops(specs, n, st);
 }
 
 void free_coldirs(ColDir* dirs) { free_colop(dirs[1].d); }
@@ -83,7 +83,7 @@ cudaError_t launch_col_pass(int pass, const PassArgs& p, const double* G, const 
   const int ntiles = (int)(a.flat ? (nx * n2 + LW - 1) / LW : a.ntx * n2);
   a.q = p.q; a.qout = p.qout; a.R = p.R; a.D = p.D; a.qsave = p.qsave; a.G = G;
   a.do_filter = p.do_filter;
-  a.c1 = p.c1; a.c2 = p.c2; a.c3 = p.c3; a.dt = p.dt;
+  a.c1 = p.c1; a.c2 = p.c2; a.c3 = p.c3; a.dt = p.dt; a.pdt = p.pdt;
   size_t smem = (size_t)2 * a.od.nch * LW * sizeof(double);
   if (pass == COL_UPDATE && p.do_filter) smem += (size_t)(p.g.N[p.dir] + 1 + 2 * COL_IMG) * LW * sizeof(double);
   return p.dir == 1 ? launch_dir<1>(pass, a, d, LW, ntiles, smem, st) : launch_dir<2>(pass, a, d, LW, ntiles, smem, st);

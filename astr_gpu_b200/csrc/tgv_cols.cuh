@@ -30,6 +30,7 @@ struct ColArgs {
   const double* G;          // fields to differentiate: 5 fluxes, or u, v, w, T
   int do_filter;
   double c1, c2, c3, dt;
+  const double* pdt;        // dt on the device when not null
 };
 
 enum ColPass { COL_FILTER = 0, COL_GRAD = 1, COL_DIV = 2, COL_UPDATE = 3 };
@@ -198,7 +199,7 @@ __device__ __forceinline__ void col_update_body(const ColArgs& a, const ColConst
   const int n0 = col_node<S>(a.od, c), nv = col_rows<S>(a.od, c);
   double* line = sm + 2 * nch * LW + COL_IMG * LW + l;   // node n at line[n * LW]
   if (act) {
-    const double c1 = a.c1, c2 = a.c2, c3 = a.c3, dt = a.dt;
+    const double c1 = a.c1, c2 = a.c2, c3 = a.c3, dt = a.pdt ? __ldg(a.pdt) : a.dt;
     // one predicated form for all chunks: a second one for whole chunks takes the kernel's code past the
     // instruction cache (512^3: 7.5 -> 9.9 ms; with range tests per row instead of is_node 5.9 -> 7.5)
     const int64_t o0 = fo + (int64_t)n0 * sd;

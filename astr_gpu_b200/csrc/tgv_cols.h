@@ -23,7 +23,7 @@ cudaError_t launch_row_c(const PassArgs& p, const RowOps& r, cudaStream_t st);
 cudaError_t launch_row_filter(const PassArgs& p, const RowOps& r, cudaStream_t st);
 
 // Directions 1 and 2 of cols[3] and the x operators, from the operators of the three directions.
-cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* cols, RowOps& rows);
+cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* cols, RowOps& rows, cudaStream_t st);
 void free_coldirs(ColDir* dirs);
 int col_lines(const ColDir& d);   // lines per CTA
 // pass: ColPass of tgv_cols.cuh (0 filter in place, 1 gradients, 2 R += D(G), 3 update and filter);

@@ -960,36 +960,6 @@ __device__ __forceinline__ void k_pass_f_body(const PassArgs& a, int bx, int by)
 }
 
 // ------------------------------------------------------------------ kernels
-// One box: the grid is the box's tile grid. Batch: blockIdx.x walks the concatenated tile grids
-// of nbox boxes (cum[k] = first CTA of box k); each CTA copies its box's arguments to shared
-// memory and runs the same body.
-struct BatchArgs {
-  const PassArgs* args;
-  const int* cum;
-  int nbox;
-};
-
-__device__ __forceinline__ const PassArgs& batch_decode(const BatchArgs& b, PassArgs& sa, int& bx, int& by) {
-  int lo = 0, hi = b.nbox - 1;
-  const int blk = blockIdx.x;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(b.cum + mid) <= blk) lo = mid;
-    else hi = mid - 1;
-  }
-  const PassArgs* src = b.args + lo;
-  const int nwords = (int)(sizeof(PassArgs) / sizeof(unsigned long long));
-  for (int w = threadIdx.x; w < nwords; w += blockDim.x)
-    reinterpret_cast<unsigned long long*>(&sa)[w] = __ldg(reinterpret_cast<const unsigned long long*>(src) + w);
-  __syncthreads();
-  const int o1 = (sa.dir == 0) ? 1 : 0;
-  const int ntx = (sa.g.N[o1] + 1 + sa.TI - 1) / sa.TI;
-  const int local = blk - __ldg(b.cum + lo);
-  by = local / ntx;
-  bx = local - by * ntx;
-  return sa;
-}
-
 // The small-box layout (3 rows per lane, one warp per line) is bounded for two 512-thread CTAs per
 // SM where that costs no more than a few spilled words (every pass but C): the boxes that use it
 // have small grids, and the SMs they fill need the second CTA to hide latency.
@@ -998,13 +968,6 @@ __device__ __forceinline__ const PassArgs& batch_decode(const BatchArgs& b, Pass
   template <TPARAMS>                                                                              \
   __global__ void __launch_bounds__(512, ASTR_MINB(S, WPL, SMALL)) NAME(PassArgs a) {             \
     NAME##_body<TARGS>(a, blockIdx.x, blockIdx.y);                                                \
-  }                                                                                               \
-  template <TPARAMS>                                                                              \
-  __global__ void __launch_bounds__(512, ASTR_MINB(S, WPL, SMALL)) NAME##_batch(BatchArgs b) {    \
-    __shared__ PassArgs sa;                                                            \
-    int bx, by;                                                                        \
-    const PassArgs& a = batch_decode(b, sa, bx, by);                                   \
-    NAME##_body<TARGS>(a, bx, by);                                                     \
   }
 
 #define ASTR_COMMA ,
@@ -1016,7 +979,7 @@ ASTR_PASS_KERNELS(k_pass_f, true, int S ASTR_COMMA int WPL ASTR_COMMA int DIR, S
 #undef ASTR_PASS_KERNELS
 #undef ASTR_COMMA
 
-// streamed forms: single-box launches only (the batched ensemble passes take all fields at once)
+// streamed forms
 #define ASTR_STREAM_KERNEL(NAME)                                         \
   template <int S, int WPL, int DIR>                                     \
   __global__ void __launch_bounds__(512, ASTR_MINB(S, WPL, true)) NAME(PassArgs a) { \
@@ -1077,34 +1040,6 @@ cudaError_t launch_pass_t(int pass, const PassArgs& a, cudaStream_t st) {
 // Dynamic shared memory of one pass launch for a tile of TI lines with pitch LP.
 inline size_t pass_smem(int pass, int TI, int LP, int WPL, int LPW, int FPS) {
   return pass_shared_bytes(pass, TI, LP, WPL, LPW, FPS);
-}
-
-template <class KernT>
-cudaError_t launch_kb(KernT kern, int nctas, int threads, size_t smem, cudaStream_t st, const BatchArgs& b) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<nctas, threads, smem, st>>>(b);
-  return cudaGetLastError();
-}
-
-// One launch of a pass over several boxes of the same solve layout (see BatchArgs).
-template <int S, int WPL>
-cudaError_t launch_pass_batch_t(int pass, int dir, const PassArgs* dargs, const int* dcum, int nbox, int nctas,
-                                int threads, size_t smem, cudaStream_t st) {
-  const BatchArgs b{dargs, dcum, nbox};
-  switch (pass) {
-    case PASS_A: return launch_kb(k_pass_ab_batch<S, WPL, DIR_A, true>, nctas, threads, smem, st, b);
-    case PASS_B: return launch_kb(k_pass_ab_batch<S, WPL, DIR_B, false>, nctas, threads, smem, st, b);
-    case PASS_C: return launch_kb(k_pass_c_batch<S, WPL, DIR_C, true>, nctas, threads, smem, st, b);
-    case PASS_VA: return launch_kb(k_pass_va_batch<S, WPL, DIR_A>, nctas, threads, smem, st, b);
-    case PASS_VB: return launch_kb(k_pass_vb_batch<S, WPL, DIR_B>, nctas, threads, smem, st, b);
-    case PASS_F:
-      if (dir == DIR_C) return launch_kb(k_pass_f_batch<S, WPL, DIR_C>, nctas, threads, smem, st, b);
-      if (dir == DIR_A) return launch_kb(k_pass_f_batch<S, WPL, DIR_A>, nctas, threads, smem, st, b);
-      return launch_kb(k_pass_f_batch<S, WPL, DIR_B>, nctas, threads, smem, st, b);
-    default:
-      return cudaErrorInvalidValue;
-  }
 }
 
 }  // namespace astr

@@ -198,9 +198,9 @@ int astr_pass_timings(astr_state* st, double dt, int nsteps, double ms[8]);
 
 /* ---- batched ensemble ---------------------------------------------------------------- */
 /* Several independent boxes (each an astr_state of the same context, sizes may differ)
- * advanced together: every pass of an RK3 stage is one launch per group of boxes sharing a
- * solve layout, and each ensemble step is one CUDA graph. No counterpart in the reference
- * (ASTR runs one block per MPI rank); the per-box results equal astr_rk3_step's. */
+ * advanced together: an ensemble step is one CUDA graph with every box's passes as a chain of
+ * their own on parallel branches; a change of the time steps keeps the graph. No counterpart in
+ * the reference (ASTR runs one block per MPI rank); the per-box results are astr_rk3_step's. */
 typedef struct astr_ensemble astr_ensemble;
 int astr_ensemble_create(astr_ctx* ctx, astr_state* const* boxes, int nbox, astr_ensemble** out);
 int astr_ensemble_destroy(astr_ensemble* e);

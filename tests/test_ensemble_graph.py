@@ -1,0 +1,36 @@
+"""The ensemble step as one graph of parallel branches: more boxes than branches, a box on lane-scan
+kernels (whose update takes the time step by value), and changes of the time steps between calls all
+give the states of the same boxes stepped alone, bit for bit (the same kernels run)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _boxes(ctx, sizes, pin=None):
+    import astr_gpu_b200 as ag
+    out = []
+    for i, n in enumerate(sizes):
+        s = ag.TGVSolver(ctx, n, params=ag.FlowParams(mach=0.2, reynolds=300.0 + 10 * i))
+        if i == pin:
+            s.set_launch_shape("B'", 3, 1, 4)
+        s.init_tgv()
+        out.append(s)
+    return out
+
+
+@pytest.mark.parametrize("sizes,pin", [([16 + k % 9 for k in range(37)], None), ([40, 16, 33, 24], 2), ([20], None)])
+def test_graph_equals_boxes_alone(sizes, pin):
+    import astr_gpu_b200 as ag
+    ctx = ag.Context(0)
+    alone, together = _boxes(ctx, sizes, pin), _boxes(ctx, sizes, pin)
+    dt = np.array([0.05 / n for n in sizes])
+    ens = ag.Ensemble(ctx, together)
+    for steps, f in ((2, 1.0), (1, 0.5), (2, 0.5), (1, 1.0)):
+        ens.step(dt * f, steps)
+        for s, d in zip(alone, dt * f):
+            s.rk3(d, steps)
+    for a, b in zip(alone, together):
+        np.testing.assert_array_equal(a.get_q(), b.get_q())
+        np.testing.assert_array_equal(a.history(), b.history())
+    ens.close()
