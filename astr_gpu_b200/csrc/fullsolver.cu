@@ -71,15 +71,17 @@ struct FsThermo {
   double mach, gamma;
 };
 
-// Node (i, j, k) of the flat index p over the box [lo[a], hi[a]] on each axis.
+// Node (i, j, k) of the flat index p over the box [lo[a], lo[a] + n[a] - 1] on each axis. Indices are
+// 32-bit (at most 1156 nodes per axis): the two 64-bit divisions per node were most of the pointwise
+// kernels' instructions. Fields of one kernel are the grid's y index.
 struct Box3 {
   int lo[3], n[3];
-  __host__ __device__ int64_t size() const { return (int64_t)n[0] * n[1] * n[2]; }
-  __device__ void node(int64_t p, int& i, int& j, int& k) const {
-    i = lo[0] + (int)(p % n[0]);
-    const int64_t r = p / n[0];
-    j = lo[1] + (int)(r % n[1]);
-    k = lo[2] + (int)(r / n[1]);
+  __host__ __device__ uint32_t size() const { return (uint32_t)n[0] * n[1] * n[2]; }
+  __device__ void node(uint32_t p, int& i, int& j, int& k) const {
+    const uint32_t r = p / (uint32_t)n[0], t = r / (uint32_t)n[1];
+    i = lo[0] + (int)(p - r * n[0]);
+    j = lo[1] + (int)(r - t * n[1]);
+    k = lo[2] + (int)t;
   }
 };
 
@@ -95,7 +97,7 @@ __host__ __device__ Box3 box_line(const FsGeo& g, int dir, int a, int b) {
 }
 
 #define GRID_STRIDE(p, total) \
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < (total); p += (int64_t)gridDim.x * blockDim.x)
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < (total); p += gridDim.x * blockDim.x)
 
 // q2fvar (fludyna.F90:545-634, tgvsolver.F90:92-121) of one node
 __device__ __forceinline__ void fs_q2fvar(const FsThermo& th, double q0, double q1, double q2, double q3, double q4,
@@ -108,17 +110,15 @@ __device__ __forceinline__ void fs_q2fvar(const FsThermo& th, double q0, double 
   t = p / rho * th.const2;
 }
 
-// Periodic halo copy along dir of nf fields (dataswap / bchomovec): F(-k) = F(N-k), F(N+k) = F(k),
+// Periodic halo copy along dir of the grid's fields (dataswap / bchomovec): F(-k) = F(N-k), F(N+k) = F(k),
 // k = 1..hm, on the lines whose other indices lie in 0..N.
-__global__ void k_fs_halo(double* F, int nf, int dir, FsGeo g) {
+__global__ void k_fs_halo(double* F, int dir, FsGeo g) {
   const Box3 b = box_line(g, dir, 1, HMW);
-  const int64_t total = b.size() * nf;
-  const int N = g.n_(dir);
+  const int N = g.n_(dir), m = blockIdx.y;
   const int64_t sd = g.s_(dir);
-  GRID_STRIDE(p, total) {
-    const int m = (int)(p / b.size());
+  GRID_STRIDE(p, b.size()) {
     int i, j, k;
-    b.node(p - (int64_t)m * b.size(), i, j, k);
+    b.node(p, i, j, k);
     const int kk = coord(dir, i, j, k);   // 1..hm
     double* f = F + m * g.fs + g.at(i, j, k) - (int64_t)kk * sd;   // node 0 of the line
     f[-(int64_t)kk * sd] = f[(int64_t)(N - kk) * sd];
@@ -133,9 +133,9 @@ __global__ void k_fs_qswap(double* q, int dir, FsGeo g) {
   const Box3 b = box_line(g, dir, 0, 0);
   const int N = g.n_(dir);
   const int64_t sd = g.s_(dir);
-  const int64_t per_line = 5 * (HMW + 1);
+  constexpr uint32_t per_line = 5 * (HMW + 1);
   GRID_STRIDE(p, b.size() * per_line) {
-    const int64_t line = p / per_line;
+    const uint32_t line = p / per_line;
     const int r = (int)(p - line * per_line);
     const int m = r / (HMW + 1), kk = r - m * (HMW + 1);
     int i, j, k;
@@ -158,9 +158,9 @@ __global__ void k_fs_qswap_prims(const double* q, double* rho, double* vel, doub
   const Box3 b = box_line(g, dir, 0, 0);
   const int N = g.n_(dir);
   const int64_t sd = g.s_(dir);
-  const int per_line = 2 * (HMW + 1);
+  constexpr uint32_t per_line = 2 * (HMW + 1);
   GRID_STRIDE(p, b.size() * per_line) {
-    const int64_t line = p / per_line;
+    const uint32_t line = p / per_line;
     const int r = (int)(p - line * per_line);
     const int t = r <= HMW ? r - HMW : N + (r - HMW - 1);   // -hm..0, then N..N+hm
     int i, j, k;
@@ -529,10 +529,10 @@ __global__ void k_fs_char_flux(double* Fh, const double* fsp, const double* fsm,
 __global__ void k_fs_flux_diff(double* qrhs, const double* Fh, int dir, FsGeo g) {
   const Box3 b = box_line(g, -1, 0, 0);
   const int64_t sd = g.s_(dir);
-  GRID_STRIDE(p, b.size() * 5) {
-    const int m = (int)(p / b.size());
+  GRID_STRIDE(p, b.size()) {
+    const int m = blockIdx.y;
     int i, j, k;
-    b.node(p - (int64_t)m * b.size(), i, j, k);
+    b.node(p, i, j, k);
     const int64_t o = m * g.fs + g.at(i, j, k);
     qrhs[o] = (qrhs[o] - Fh[o]) + Fh[o - sd];
   }
@@ -546,10 +546,10 @@ __global__ void k_fs_mp_flux(double* Fh, const double* fsp, const double* fsm, c
   const int N = g.n_(dir);
   const Box3 b = box_line(g, dir, -1, N);
   const int64_t sd = g.s_(dir);
-  GRID_STRIDE(p, b.size() * 5) {
-    const int m = (int)(p / b.size());
+  GRID_STRIDE(p, b.size()) {
+    const int m = blockIdx.y;
     int i, j, k;
-    b.node(p - (int64_t)m * b.size(), i, j, k);
+    b.node(p, i, j, k);
     const int t = dir == 0 ? i : (dir == 1 ? j : k);
     const int64_t o = m * g.fs + g.at(i, j, k);
     Fh[o] = fs_interface(fsp, fsm, fhp, fhm, o - (int64_t)t * sd, sd, t, N, nt, iss, iee);
@@ -614,10 +614,10 @@ __global__ void k_fs_update(double* q, double* qsave, const double* qrhs, double
                             int first, FsGeo g) {
   const Box3 b = box_line(g, -1, 0, 0);
   const double jb = g.jac;
-  GRID_STRIDE(p, b.size() * 5) {
-    const int m = (int)(p / b.size());
+  GRID_STRIDE(p, b.size()) {
+    const int m = blockIdx.y;
     int i, j, k;
-    b.node(p - (int64_t)m * b.size(), i, j, k);
+    b.node(p, i, j, k);
     const int64_t o = m * g.fs + g.at(i, j, k);
     if (first) qsave[o] = q[o] * jb;
     const double v = c1 * qsave[o] + c2 * q[o] * jb + c3 * qrhs[o] * dt;
@@ -681,12 +681,12 @@ __global__ void k_fs_diag(double* partials, const double* rho, const double* vel
 // Copy between the caller's Fortran array (nodes 0..N inside it) and nodes 0..N of the layout,
 // nf fields.
 __global__ void k_fs_pack(double* state, double* user, FsGeo g, int64_t u0, int64_t u1, int64_t u2, int64_t ufs,
-                          int64_t uoff, int to_state, int nf) {
+                          int64_t uoff, int to_state) {
   const Box3 b = box_line(g, -1, 0, 0);
-  GRID_STRIDE(p, b.size() * nf) {
-    const int m = (int)(p / b.size());
+  GRID_STRIDE(p, b.size()) {
+    const int m = blockIdx.y;
     int i, j, k;
-    b.node(p - (int64_t)m * b.size(), i, j, k);
+    b.node(p, i, j, k);
     const int64_t os = m * g.fs + g.at(i, j, k);
     const int64_t ou = uoff + m * ufs + i * u0 + j * u1 + k * u2;
     if (to_state) state[os] = user[ou];
@@ -813,12 +813,12 @@ cudaError_t fs_convection_upwind(astr_full* fs) {
       k_fs_char_flux<<<blocks_for(ni), 256, 0, st>>>(fs->work, fsp, fsm, fhp, fhm, fs->q, fs->rho, fs->vel, fs->prs,
                                                      lsh, d, nt, iss, iee, g, fs->th);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      k_fs_flux_diff<<<blocks_for(5 * nn), 256, 0, st>>>(fs->qrhs, fs->work, d, g);
+      k_fs_flux_diff<<<dim3(blocks_for(nn), 5), 256, 0, st>>>(fs->qrhs, fs->work, d, g);
     } else {
       const int64_t ni = nn / (g.N[d] + 1) * (g.N[d] + 2);
-      k_fs_mp_flux<<<blocks_for(5 * ni), 256, 0, st>>>(fs->work, fsp, fsm, fhp, fhm, d, nt, iss, iee, g);
+      k_fs_mp_flux<<<dim3(blocks_for(ni), 5), 256, 0, st>>>(fs->work, fsp, fsm, fhp, fhm, d, nt, iss, iee, g);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      k_fs_flux_diff<<<blocks_for(5 * nn), 256, 0, st>>>(fs->qrhs, fs->work, d, g);
+      k_fs_flux_diff<<<dim3(blocks_for(nn), 5), 256, 0, st>>>(fs->qrhs, fs->work, d, g);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -826,8 +826,8 @@ cudaError_t fs_convection_upwind(astr_full* fs) {
 }
 
 cudaError_t fs_halo(astr_full* fs, double* F, int nf, int dir) {
-  const int64_t n = (int64_t)nf * HMW * (fs->g.N[0] + 1) * (fs->g.N[1] + 1) * (fs->g.N[2] + 1) / (fs->g.n_(dir) + 1);
-  k_fs_halo<<<blocks_for(n), 256, 0, astr_ctx_stream(fs->ctx)>>>(F, nf, dir, fs->g);
+  const int64_t n = (int64_t)HMW * (fs->g.N[0] + 1) * (fs->g.N[1] + 1) * (fs->g.N[2] + 1) / (fs->g.n_(dir) + 1);
+  k_fs_halo<<<dim3(blocks_for(n), nf), 256, 0, astr_ctx_stream(fs->ctx)>>>(F, dir, fs->g);
   return cudaGetLastError();
 }
 
@@ -912,7 +912,7 @@ cudaError_t fs_step(astr_full* fs, double dt) {
   cudaError_t e;
   for (int s = 0; s < 3; ++s) {
     if ((e = fs_stage_rhs(fs, s == 0)) != cudaSuccess) return e;
-    k_fs_update<<<blocks_for(5 * nn), 256, 0, st>>>(fs->q, fs->qsave, fs->qrhs, rk[s][0], rk[s][1], rk[s][2], dt,
+    k_fs_update<<<dim3(blocks_for(nn), 5), 256, 0, st>>>(fs->q, fs->qsave, fs->qrhs, rk[s][0], rk[s][1], rk[s][2], dt,
                                                    s == 0, fs->g);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_fs_prims<<<blocks_for(nn), 256, 0, st>>>(fs->q, fs->rho, fs->vel, fs->prs, fs->tmp, fs->g, fs->th);
@@ -946,7 +946,7 @@ int fs_copy(astr_full* fs, double* user, const int64_t* shape, const int64_t* lb
       FCK(cudaMemcpyAsync(dev, user, bytes, cudaMemcpyHostToDevice, st));
     }
   }
-  k_fs_pack<<<blocks_for(5 * nodes(fs)), 256, 0, st>>>(fs->q, dev, fs->g, 1, u1, u2, ufs, uoff, to_state, 5);
+  k_fs_pack<<<dim3(blocks_for(nodes(fs)), 5), 256, 0, st>>>(fs->q, dev, fs->g, 1, u1, u2, ufs, uoff, to_state);
   FCK(cudaGetLastError());
   if (where == ASTR_HOST && !to_state) {
     // the staging buffer holds the caller's layout with only nodes 0..N written: an array with
@@ -1132,7 +1132,7 @@ int astr_full_write_flowfield(astr_full* fs, const char* filename) {
   const int64_t shape[3] = {fs->p.im + 1, fs->p.jm + 1, fs->p.km + 1};
   const int64_t n = shape[0] * shape[1] * shape[2];
   double* dprims = fs->dvel;   // 9 layout fields, free between steps
-  k_fs_pack<<<blocks_for(6 * n), 256, 0, st>>>(fs->rho, dprims, fs->g, 1, shape[0], shape[0] * shape[1], n, 0, 0, 6);
+  k_fs_pack<<<dim3(blocks_for(n), 6), 256, 0, st>>>(fs->rho, dprims, fs->g, 1, shape[0], shape[0] * shape[1], n, 0, 0);
   cudaError_t e = cudaGetLastError();
   std::string err;
   int rc = e != cudaSuccess ? ASTR_ERR_CUDA : flowfield_write(st, dprims, shape, fs->nstep, fs->time, filename, err);
@@ -1164,7 +1164,7 @@ int astr_full_read_flowfield(astr_full* fs, const char* filename, char mode, int
   if (rc == ASTR_OK) {
     rc = astr_full_upload(fs, dq, shape, lb, ASTR_DEVICE);   // sets the context's message on failure
     if (rc == ASTR_OK) {
-      k_fs_pack<<<blocks_for(6 * n), 256, 0, st>>>(fs->rho, dprims, fs->g, 1, shape[0], shape[0] * shape[1], n, 0, 1, 6);
+      k_fs_pack<<<dim3(blocks_for(n), 6), 256, 0, st>>>(fs->rho, dprims, fs->g, 1, shape[0], shape[0] * shape[1], n, 0, 1);
       if ((e = cudaGetLastError()) == cudaSuccess) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) {
         rc = ASTR_ERR_CUDA;
