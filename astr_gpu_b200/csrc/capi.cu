@@ -226,8 +226,13 @@ int line_call(astr_ctx* ctx, const astr_scheme* s, int dir, const double* f, con
 int scheme_tables(astr_ctx* ctx, astr_scheme* s, astr_scheme** out) {
   const int nsys = s->h.nsys();
   if (col_rows_per_chunk(nsys, 0) == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
-  const ColSpec specs[2] = {{&s->h, col_rows_per_chunk(nsys, 0), 0, &s->d[0]}, {&s->h, col_rows_per_chunk(nsys, 1), 0, &s->d[1]}};
-  const cudaError_t e = make_colops(specs, 2, ctx->stream);
+  const int sx = col_rows_per_chunk(nsys, 0), sy = col_rows_per_chunk(nsys, 1);
+  const ColSpec specs[2] = {{&s->h, sx, 0, &s->d[0]}, {&s->h, sy, 0, &s->d[1]}};
+  const cudaError_t e = make_colops(specs, sx == sy ? 1 : 2, ctx->stream);
+  if (sx == sy) {   // one table serves all directions
+    s->d[1] = s->d[0];
+    s->d[1].dtab = nullptr;
+  }
   if (e != cudaSuccess) {
     free_colop(s->d[0]);
     delete s;

@@ -287,10 +287,15 @@ static cudaError_t launch_sk(const DevColOp& op, const LineArgs& a, int nfields,
     if constexpr (S >= 33) return launch_col<S, KIND, 16>(op, a, nfields, st);
     return cudaErrorInvalidValue;
   }
-  constexpr int LW = 16;
+  // long chunks: 8 lines with a pitch of 2 mod 16 (a half warp is 8 lines on the even bank pairs and the
+  // next chunk, an odd number of rows away, on the odd ones), several small CTAs per SM; else 16 lines
+  // with an odd pitch. GB/s with 16 / 8 lines: derivative 512 nodes 3715 / 3919, filter 512 nodes 3362 /
+  // 3514, 1050 nodes 2314 / 2726, 256 nodes 3339 / 3395
+  constexpr int LW = S >= 33 ? 8 : 16;
   const int threads = (op.op.nch * LW + 31) / 32 * 32;
   const dim3 grid((unsigned)((a.oa.n[1] + LW - 1) / LW), (unsigned)a.oa.n[2], (unsigned)nfields);
-  const int LP = (op.line.dim + 1 + 2 * HL) | 1;
+  const int need = op.line.dim + 1 + 2 * HL;
+  const int LP = LW == 8 ? need + (18 - need % 16) % 16 : need | 1;
   const size_t smem = ((size_t)2 * op.op.nch * LW + (size_t)LW * LP) * sizeof(double);
   auto kern = k_line_row<S, KIND, LW>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
