@@ -24,6 +24,7 @@
 // compact flux of each split part (flux_uw/flux_dw, src/flux.F90:125-150), the MP limiter at
 // every interface (shock = .true. with no Ducros sensor, crinod .false.), and the flux
 // difference added to qrhs.
+#include <algorithm>
 #include <cmath>
 #include <new>
 #include <string>
@@ -472,8 +473,10 @@ __global__ void k_fs_lshock(double* lsh, const double* ssf, double shkcrt, FsGeo
 // one thread per interface i = -1..N of a line, all five components: the split fluxes of the
 // iwind6 stencils and the compact fluxes projected on the left eigenvectors, the MP limiter in
 // characteristic variables with the interface's shock flag, back by the right eigenvectors.
-// Fh(i) is stored at node i of the layout (work fields).
-__global__ void k_fs_char_flux(double* Fh, const double* fsp, const double* fsm, const double* fhp, const double* fhm,
+// Fh(i) is stored at node i of the layout (work fields). Latency bounds it: 12 warps per SM at 168
+// registers (a few spilled words) beat 8 at 255 with every stencil read five times (a whole 96^3 step
+// 4.62 -> 4.51 ms) and 8 at 196 without spills (4.69 against 4.46 ms, another run).
+__global__ void __launch_bounds__(128, 3) k_fs_char_flux(double* Fh, const double* fsp, const double* fsm, const double* fhp, const double* fhm,
                                const double* q, const double* rho, const double* vel, const double* prs,
                                const double* lsh, int dir, int nt, int iss, int iee, FsGeo g, FsThermo th) {
   const int N = g.n_(dir);
@@ -492,31 +495,42 @@ __global__ void k_fs_char_flux(double* Fh, const double* fsp, const double* fsm,
     else shock = lsh[oa] != 0.0 || lsh[ob] != 0.0;
     const double vl[3] = {vel[oa], vel[fs + oa], vel[2 * fs + oa]};
     const double vr[3] = {vel[ob], vel[fs + ob], vel[2 * fs + ob]};
-    double R[5][5], L[5][5];
-    fs_chardecomp(th, rho[oa], prs[oa], q[4 * fs + oa], vl, rho[ob], prs[ob], q[4 * fs + ob], vr, mrow, R, L);
-    int64_t jp[5], jn[5];
-#pragma unroll
-    for (int n = 1; n <= 5; ++n) {
-      jp[n - 1] = o0 + (int64_t)min(max(t + n - 3, iss), iee) * sd;
-      jn[n - 1] = o0 + (int64_t)min(max(t + 4 - n, iss), iee) * sd;
-    }
+    const double ra = rho[oa], pa = prs[oa], ea = q[4 * fs + oa], rb = rho[ob], pb = prs[ob], eb = q[4 * fs + ob];
     double fhc[5];
+    {
+      double R[5][5], L[5][5];
+      fs_chardecomp(th, ra, pa, ea, vl, rb, pb, eb, vr, mrow, R, L);
+      // one side after the other: its 25 stencil values are loaded once for the five characteristics
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      double up[5], um[5];
+      for (int side = 0; side < 2; ++side) {
+        const double* f = side == 0 ? fsp : fsm;
+        const double* fh = side == 0 ? fhp : fhm;
+        double x[5][5], h[5];
 #pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        up[n] = L[m][0] * fsp[jp[n]] + L[m][1] * fsp[fs + jp[n]] + L[m][2] * fsp[2 * fs + jp[n]] +
-                L[m][3] * fsp[3 * fs + jp[n]] + L[m][4] * fsp[4 * fs + jp[n]];
-        um[n] = L[m][0] * fsm[jn[n]] + L[m][1] * fsm[fs + jn[n]] + L[m][2] * fsm[2 * fs + jn[n]] +
-                L[m][3] * fsm[3 * fs + jn[n]] + L[m][4] * fsm[4 * fs + jn[n]];
+        for (int n = 1; n <= 5; ++n) {
+          const int64_t o = o0 + (int64_t)min(max(side == 0 ? t + n - 3 : t + 4 - n, iss), iee) * sd;
+#pragma unroll
+          for (int c = 0; c < 5; ++c) x[n - 1][c] = f[c * fs + o];
+        }
+#pragma unroll
+        for (int c = 0; c < 5; ++c) h[c] = fh[c * fs + oa];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          double u[5];
+#pragma unroll
+          for (int n = 0; n < 5; ++n)
+            u[n] = L[m][0] * x[n][0] + L[m][1] * x[n][1] + L[m][2] * x[n][2] + L[m][3] * x[n][3] + L[m][4] * x[n][4];
+          const double v = fs_mplimiter(u, L[m][0] * h[0] + L[m][1] * h[1] + L[m][2] * h[2] + L[m][3] * h[3] + L[m][4] * h[4],
+                                        shock, t, N, nt);
+          fhc[m] = side == 0 ? v : fhc[m] + v;
+        }
       }
-      const double hp = L[m][0] * fhp[oa] + L[m][1] * fhp[fs + oa] + L[m][2] * fhp[2 * fs + oa] +
-                        L[m][3] * fhp[3 * fs + oa] + L[m][4] * fhp[4 * fs + oa];
-      const double hm = L[m][0] * fhm[oa] + L[m][1] * fhm[fs + oa] + L[m][2] * fhm[2 * fs + oa] +
-                        L[m][3] * fhm[3 * fs + oa] + L[m][4] * fhm[4 * fs + oa];
-      fhc[m] = fs_mplimiter(up, hp, shock, t, N, nt) + fs_mplimiter(um, hm, shock, t, N, nt);
     }
+    // the right eigenvectors are formed anew: kept beside the left ones and the stencils they would spill
+    double rc = ra;
+    asm volatile("" : "+d"(rc));
+    double R[5][5], L[5][5];
+    fs_chardecomp(th, rc, pa, ea, vl, rb, pb, eb, vr, mrow, R, L);
 #pragma unroll
     for (int m = 0; m < 5; ++m)
       Fh[m * fs + oa] = R[m][0] * fhc[0] + R[m][1] * fhc[1] + R[m][2] * fhc[2] + R[m][3] * fhc[3] + R[m][4] * fhc[4];
@@ -810,7 +824,7 @@ cudaError_t fs_convection_upwind(astr_full* fs) {
     if ((e = flux_op(fs, fs->dfd[d], d, fsm, fhm, 5)) != cudaSuccess) return e;
     if (fs->p.lchardecomp) {
       const int64_t ni = nn / (g.N[d] + 1) * (g.N[d] + 2);
-      k_fs_char_flux<<<blocks_for(ni), 256, 0, st>>>(fs->work, fsp, fsm, fhp, fhm, fs->q, fs->rho, fs->vel, fs->prs,
+      k_fs_char_flux<<<(unsigned)std::min<int64_t>((ni + 127) / 128, 148 * 24), 128, 0, st>>>(fs->work, fsp, fsm, fhp, fhm, fs->q, fs->rho, fs->vel, fs->prs,
                                                      lsh, d, nt, iss, iee, g, fs->th);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       k_fs_flux_diff<<<dim3(blocks_for(nn), 5), 256, 0, st>>>(fs->qrhs, fs->work, d, g);
