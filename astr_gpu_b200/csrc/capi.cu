@@ -76,8 +76,8 @@ struct astr_state {
 struct astr_ensemble {
   astr_ctx* ctx = nullptr;
   std::vector<astr_state*> boxes;
-  std::vector<double> dt;
-  double* ddt = nullptr;            // the boxes' time steps on the device
+  std::vector<double> dt;           // the time steps that ddt holds
+  double* ddt = nullptr;            // the boxes' time steps on the device, read by every box's update
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};   // filter along A owed at the start of the step or not
   bool pending = false;
 };
@@ -1289,14 +1289,15 @@ int astr_ensemble_step(astr_ensemble* e, const double* dt, int nsteps) {
   if (!all_pending)
     for (int b = 0; b < nbox; ++b) CK(finalize_filter(e->boxes[b]));
   e->pending = all_pending;
-  if (changed) {
-    e->dt.assign(dt, dt + nbox);
-    CK(cudaMemcpyAsync(e->ddt, dt, (size_t)nbox * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  if (changed) {   // e->dt is what the device holds: set once the copy is queued
+    std::vector<double> now(dt, dt + nbox);
+    e->dt.clear();
+    CK(cudaMemcpyAsync(e->ddt, now.data(), (size_t)nbox * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    e->dt = std::move(now);
   }
   for (int b = 0; b < nbox && nsteps > 0; ++b) {
     astr_state* st = e->boxes[b];
     if (wants_tuning(st)) CK(autotune(st));
-    if (changed && !st->use_col[CFG_VB]) ens_drop_graphs(e);   // its update takes the time step by value
   }
   for (int s = 0; s < nsteps; ++s) {
     const int variant = e->pending ? 1 : 0;

@@ -798,7 +798,7 @@ __device__ __forceinline__ void k_pass_vbs_body(const PassArgs& a, int bx, int b
     }
     // SSP-RK3 stage update of the group's fields, with the periodic images for the filter
     if (c.svalid) {
-      const double c1 = a.c1, c2 = a.c2, c3 = a.c3, dt = a.dt;
+      const double c1 = a.c1, c2 = a.c2, c3 = a.c3, dt = a.pdt ? __ldg(a.pdt) : a.dt;
 #pragma unroll 1
       for (int j = 0; j < cnt; ++j) {
         double* Tm = T + j * tsz;
@@ -904,7 +904,7 @@ __device__ __forceinline__ void k_pass_vb_body(const PassArgs& a, int bx, int by
   // SSP-RK3 stage update of every field, with the periodic images for the filter
   const int dim = c.dim;
   if (c.svalid) {
-    const double c1 = a.c1, c2 = a.c2, c3 = a.c3, dt = a.dt;
+    const double c1 = a.c1, c2 = a.c2, c3 = a.c3, dt = a.pdt ? __ldg(a.pdt) : a.dt;
     const double* qs = a.qsave + c.sbase;
     const double* qq = a.q + c.sbase;
     const double* R = a.R + c.sbase;

@@ -30,7 +30,27 @@ def test_graph_equals_boxes_alone(sizes, pin):
         ens.step(dt * f, steps)
         for s, d in zip(alone, dt * f):
             s.rk3(d, steps)
+    _equal(alone, together)
+    ens.close()
+
+
+def _equal(alone, together):
     for a, b in zip(alone, together):
         np.testing.assert_array_equal(a.get_q(), b.get_q())
         np.testing.assert_array_equal(a.history(), b.history())
+
+
+def test_time_steps_changed_by_a_call_of_no_steps():
+    """The new time steps reach every box also when the call that brings them makes no step."""
+    import astr_gpu_b200 as ag
+    ctx = ag.Context(0)
+    sizes = [24, 16, 40]
+    alone, together = _boxes(ctx, sizes, 0), _boxes(ctx, sizes, 0)
+    dt = np.array([0.05 / n for n in sizes])
+    ens = ag.Ensemble(ctx, together)
+    for steps, f in ((2, 1.0), (0, 0.5), (1, 0.5), (0, 2.0), (0, 0.25), (2, 0.25)):
+        ens.step(dt * f, steps)
+        for s, d in zip(alone, dt * f):
+            s.rk3(d, steps)
+    _equal(alone, together)
     ens.close()
