@@ -71,6 +71,7 @@ struct astr_state {
   bool use_graph = true;
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   double gdt[2] = {0.0, 0.0};
+  unsigned config = 0;        // counts the changes of the passes' launch configuration
 };
 
 struct astr_ensemble {
@@ -79,6 +80,7 @@ struct astr_ensemble {
   std::vector<double> dt;           // the time steps that ddt holds
   double* ddt = nullptr;            // the boxes' time steps on the device, read by every box's update
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};   // filter along A owed at the start of the step or not
+  std::vector<unsigned> config;     // the boxes' launch configurations that the graphs hold
   bool pending = false;
 };
 
@@ -587,7 +589,10 @@ bool wants_tuning(const astr_state* st) {
   return st->autotune && !st->tuned && lanes;
 }
 
+// After a change of the passes' launch configuration: the state's own graphs go, an ensemble that has
+// captured the state sees the count.
 void drop_graphs(astr_state* st) {
+  ++st->config;
   for (auto& g : st->gexec)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
@@ -1297,7 +1302,16 @@ int astr_ensemble_step(astr_ensemble* e, const double* dt, int nsteps) {
   }
   for (int b = 0; b < nbox && nsteps > 0; ++b) {
     astr_state* st = e->boxes[b];
-    if (wants_tuning(st)) CK(autotune(st));
+    if (wants_tuning(st)) {
+      drop_graphs(st);
+      CK(autotune(st));
+    }
+  }
+  std::vector<unsigned> config;
+  for (astr_state* st : e->boxes) config.push_back(st->config);
+  if (config != e->config) {
+    ens_drop_graphs(e);
+    e->config = std::move(config);
   }
   for (int s = 0; s < nsteps; ++s) {
     const int variant = e->pending ? 1 : 0;

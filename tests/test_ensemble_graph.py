@@ -54,3 +54,22 @@ def test_time_steps_changed_by_a_call_of_no_steps():
             s.rk3(d, steps)
     _equal(alone, together)
     ens.close()
+
+
+@pytest.mark.parametrize("change", [lambda s: s.set_launch_shape("A'", 3, 1, 4), lambda s: s.split_filter(False)])
+def test_shapes_changed_after_the_first_step(change):
+    """A box's passes run in the form it is set to, also when the ensemble has stepped it before."""
+    import astr_gpu_b200 as ag
+    ctx = ag.Context(0)
+    sizes = [24, 33]
+    alone, together = _boxes(ctx, sizes), _boxes(ctx, sizes)
+    dt = np.array([0.05 / n for n in sizes])
+    ens = ag.Ensemble(ctx, together)
+    for _ in range(2):
+        ens.step(dt, 3)
+        for s, d in zip(alone, dt):
+            s.rk3(d, 3)
+        change(alone[1])
+        change(together[1])
+    _equal(alone, together)
+    ens.close()
