@@ -1071,12 +1071,14 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
       add(fs->hfu[d], fs->dfu[d]);
       add(fs->hfd[d], fs->dfd[d]);
     }
-    if (col_rows_per_chunk(fs->hf[d].nsys(), d) == 0) {
+  }
+  // the longest system decides: the filter's, or between two walls the interface flux's (N + 2 rows)
+  for (const ColSpec& s : specs)
+    if (s.S == 0) {
       delete fs;
-      astr_ctx_set_error(ctx, "dimension too large (max 1145)");
+      astr_ctx_set_error(ctx, "dimension too large: a line system of more than 1152 rows (periodic directions take 1145)");
       return ASTR_ERR_UNSUPPORTED;
     }
-  }
   if (make_colops(specs.data(), (int)specs.size(), astr_ctx_stream(ctx)) != cudaSuccess) {
     astr_full_destroy(fs);
     astr_ctx_set_error(ctx, "scheme tables");

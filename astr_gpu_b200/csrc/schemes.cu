@@ -326,11 +326,11 @@ int col_rows_per_chunk(int nsys, int dir) {
 // embeds an operator in the chunks of one with a longer system).
 // The host side of make_colop: everything but the device copy of the table `t`.
 static cudaError_t fill_colop(const HostOp& h, int S, int pad, DevColOp& out, std::vector<double>& t) {
+  const int n0 = h.nsys(), nsys = n0 + 2 * pad;
+  if (S < 1 || S > COL_MAXS || nsys < 2 * S) return cudaErrorInvalidValue;
   fill_lineop(h, out.line);
   out.S = S;
-  const int n0 = h.nsys(), nsys = n0 + 2 * pad;
   const int nch = std::max(3, (nsys + S - 1) / S);
-  if (nsys < 2 * S) return cudaErrorInvalidValue;
   ColOp& o = out.op;
   o.nch = nch;
   o.nv = nsys - (nch - 1) * S;
@@ -372,7 +372,7 @@ static cudaError_t fill_colop(const HostOp& h, int S, int pad, DevColOp& out, st
     if (o.c_lo % 2 == 0) ++o.c_lo;   // with the last one an even number of table chunks
     o.c_lo = std::min(o.c_lo, nch - 1);
   }
-  for (int k = 0; k < S && S <= COL_MAXS; ++k) { out.pf[k] = tr[6 * k + 2]; out.qb[k] = tr[6 * k + 4]; }
+  for (int k = 0; k < S; ++k) { out.pf[k] = tr[6 * k + 2]; out.qb[k] = tr[6 * k + 4]; }
   out.k3 = tr[1];
   out.k1 = tr[3];
   out.k2 = flat ? tr[0] : 1.0;

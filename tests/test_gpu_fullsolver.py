@@ -350,6 +350,25 @@ def test_full_solver_rejects_bad_parameters(ctx):
         assert e.value.code == -1, kw
 
 
+def test_longest_lines_between_walls(ctx):
+    """Between two walls the filter's system has N + 1 rows and the interface flux's N + 2, at most 1152:
+    N = 1151 runs with the central scheme and is refused with the upwind one, which takes 1150."""
+    import astr_gpu_b200 as ag
+    for n, sch in ((1151, 643), (1150, 543)):
+        dims = (16, 16, n)
+        s = ag.FullSolver(ctx, *dims, params=ag.FlowParams(mach=0.3, conschm=sch, ntype=(3, 3, 4), twall=1.0))
+        q = np.zeros(tuple(d + 1 for d in dims) + (5,), order="F")
+        q[..., 0] = 1.0
+        q[..., 4] = 1.0 / (1.4 * 0.09) / 0.4
+        s.set_q(q)
+        assert np.abs(s.rhs()).max() <= 1e-10   # a gas at rest
+        s.close()
+    for n, sch in ((1151, 543), (1152, 543), (1152, 643)):
+        with pytest.raises(ag.AstrError) as e:
+            ag.FullSolver(ctx, 16, 16, n, params=ag.FlowParams(mach=0.3, conschm=sch, ntype=(3, 3, 4)))
+        assert e.value.code == -4
+
+
 def test_characteristic_mode_rejects_walls(ctx):
     import astr_gpu_b200 as ag
     with pytest.raises(ag.AstrError) as e:
