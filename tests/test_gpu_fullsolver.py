@@ -356,12 +356,13 @@ def test_longest_lines_between_walls(ctx):
     import astr_gpu_b200 as ag
     for n, sch in ((1151, 643), (1150, 543)):
         dims = (16, 16, n)
-        s = ag.FullSolver(ctx, *dims, params=ag.FlowParams(mach=0.3, conschm=sch, ntype=(3, 3, 4), twall=1.0))
+        p = ag.FlowParams(mach=0.3, conschm=sch, ntype=(3, 3, 4), twall=1.0, beta_bound=0.98)
+        s = ag.FullSolver(ctx, *dims, params=p)
         q = np.zeros(tuple(d + 1 for d in dims) + (5,), order="F")
         q[..., 0] = 1.0
         q[..., 4] = 1.0 / (1.4 * 0.09) / 0.4
         s.set_q(q)
-        assert np.abs(s.rhs()).max() <= 1e-10   # a gas at rest
+        assert np.abs(s.rhs()).max() <= 1e-10   # a gas at rest (at beta_bound 0.98 the filter keeps constants)
         s.close()
     for n, sch in ((1151, 543), (1152, 543), (1152, 643)):
         with pytest.raises(ag.AstrError) as e:
