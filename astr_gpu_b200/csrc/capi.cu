@@ -22,6 +22,7 @@ struct astr_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  cudaStream_t setup = nullptr;   // operators' tables reach the device here: nothing else to wait for
   std::string err;
   double* stage = nullptr;     // device staging of the line calls on host arrays (grows, kept)
   size_t stage_bytes = 0;
@@ -229,8 +230,8 @@ int scheme_tables(astr_ctx* ctx, astr_scheme* s, astr_scheme** out) {
   const int nsys = s->h.nsys();
   if (col_rows_per_chunk(nsys, 0) == 0) { delete s; return fail(ctx, ASTR_ERR_UNSUPPORTED, "line longer than 1152 rows"); }
   const int sx = col_rows_per_chunk(nsys, 0), sy = col_rows_per_chunk(nsys, 1);
-  const ColSpec specs[2] = {{&s->h, sx, 0, &s->d[0]}, {&s->h, sy, 0, &s->d[1]}};
-  const cudaError_t e = make_colops(specs, sx == sy ? 1 : 2, ctx->stream);
+  ColSpec specs[2] = {{&s->h, sx, 0, &s->d[0]}, {&s->h, sy, 0, &s->d[1]}};
+  const cudaError_t e = make_colops(specs, sx == sy ? 1 : 2, ctx->setup);
   if (sx == sy) {   // one table serves all directions
     s->d[1] = s->d[0];
     s->d[1].dtab = nullptr;
@@ -601,6 +602,7 @@ void drop_graphs(astr_state* st) {
 
 // Used by noalloc.cu.
 cudaStream_t astr_ctx_stream(astr_ctx* ctx) { return ctx->stream; }
+cudaStream_t astr_ctx_setup_stream(astr_ctx* ctx) { return ctx->setup; }
 int astr_ctx_device(astr_ctx* ctx) { return ctx->device; }
 void astr_ctx_set_error(astr_ctx* ctx, const char* msg) { ctx->err = msg; }
 
@@ -618,6 +620,11 @@ int astr_init(int device, astr_ctx** out) {
   c->device = device;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return ASTR_ERR_CUDA; }
   c->own_stream = true;
+  if (cudaStreamCreateWithFlags(&c->setup, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaStreamDestroy(c->stream);
+    delete c;
+    return ASTR_ERR_CUDA;
+  }
   *out = c;
   return ASTR_OK;
 }
@@ -630,6 +637,7 @@ int astr_destroy(astr_ctx* c) {
     cudaFree(c->stage);
   }
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
+  if (c->setup) cudaStreamDestroy(c->setup);
   delete c;
   return ASTR_OK;
 }
@@ -792,15 +800,18 @@ int astr_state_create(astr_ctx* ctx, const astr_params* p, astr_state** out) {
     c.TI = pick_ti(pass_tiles(CFG_PASS[id]), N[d], L.WPL, L.S);
     c.LP = tile_pitch(N[d], c.TI, c.S);
   }
-  const cudaError_t ec = make_coldirs(st->hd, st->hf, st->col, st->rows, ctx->stream);
+  std::vector<ColSpec> specs;
+  std::vector<double> tab;
+  const cudaError_t ec = fill_coldirs(st->hd, st->hf, st->col, st->rows, specs, tab);
   if (ec != cudaSuccess) { astr_state_destroy(st); return cuda_fail(ctx, ec, "column operators"); }
   st->use_col[CFG_C] = st->rows.c.S != 0;
   st->use_col[CFG_FC] = st->rows.f.S != 0;
   // a small box gains nothing from tuning
   st->autotune = (N[0] + 1) * (int64_t)(N[1] + 1) * (N[2] + 1) >= 100 * 100 * 100;
-  // 33 fields: Q0(5) Q1(5) R(5) DA(4) DB(4) VF(10: the combined fluxes along A and along B)
+  // 33 fields: Q0(5) Q1(5) R(5) DA(4) DB(4) VF(10: the combined fluxes along A and along B), then the
+  // column operators' table
   const size_t nf = 33;
-  cudaError_t e = cudaMalloc(&st->buf, nf * (size_t)st->g.fs * sizeof(double));
+  cudaError_t e = cudaMalloc(&st->buf, (nf * (size_t)st->g.fs + tab.size()) * sizeof(double));
   if (e != cudaSuccess) { astr_state_destroy(st); return fail(ctx, ASTR_ERR_NOMEM, "state allocation"); }
   cudaMemsetAsync(st->buf, 0, nf * (size_t)st->g.fs * sizeof(double), ctx->stream);
   st->Q0 = st->buf;
@@ -809,6 +820,10 @@ int astr_state_create(astr_ctx* ctx, const astr_params* p, astr_state** out) {
   st->DA = st->R + 5 * st->g.fs;
   st->DB = st->DA + 4 * st->g.fs;
   st->VF = st->DB + 4 * st->g.fs;
+  if ((e = load_colops(specs.data(), (int)specs.size(), tab, st->buf + nf * st->g.fs, ctx->setup)) != cudaSuccess) {
+    astr_state_destroy(st);
+    return cuda_fail(ctx, e, "column operators");
+  }
   // partial sums of pass C: one per CTA
   const int o1 = (DIR_C == 0) ? 1 : 0, o2 = (DIR_C == 2) ? 1 : 2;
   st->nparts = (int)((N[o1] + 1) * (int64_t)(N[o2] + 1));   // one per CTA; at least one line per CTA
@@ -829,7 +844,6 @@ int astr_state_destroy(astr_state* st) {
   if (!st) return ASTR_ERR_ARG;
   drop_graphs(st);
   for (auto& kv : st->ops) { free_devop(kv.second.first); free_devop(kv.second.second); }
-  free_coldirs(st->col);
   if (st->buf) cudaFree(st->buf);
   if (st->partials) cudaFree(st->partials);
   if (st->hist) cudaFree(st->hist);

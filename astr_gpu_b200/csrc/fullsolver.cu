@@ -38,6 +38,7 @@ using namespace astr;
 
 // Defined in capi.cu.
 cudaStream_t astr_ctx_stream(astr_ctx* ctx);
+cudaStream_t astr_ctx_setup_stream(astr_ctx* ctx);
 int astr_ctx_device(astr_ctx* ctx);
 void astr_ctx_set_error(astr_ctx* ctx, const char* msg);
 
@@ -1079,7 +1080,7 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
       astr_ctx_set_error(ctx, "dimension too large: a line system of more than 1152 rows (periodic directions take 1145)");
       return ASTR_ERR_UNSUPPORTED;
     }
-  if (make_colops(specs.data(), (int)specs.size(), astr_ctx_stream(ctx)) != cudaSuccess) {
+  if (make_colops(specs.data(), (int)specs.size(), astr_ctx_setup_stream(ctx)) != cudaSuccess) {
     astr_full_destroy(fs);
     astr_ctx_set_error(ctx, "scheme tables");
     return ASTR_ERR_CUDA;

@@ -66,8 +66,13 @@ struct ColSpec {
   const HostOp* h;
   int S, pad;      // rows per chunk, identity rows around the system
   DevColOp* out;
+  size_t at = 0;   // its part of the common table
 };
-cudaError_t make_colops(const ColSpec* specs, int n, cudaStream_t st);   // one allocation, freed with the first
+// Operators and their common table: filled on the host, then copied to `dev` on a stream that holds
+// nothing else (the call returns when the copy is done).
+cudaError_t fill_colops(ColSpec* specs, int n, std::vector<double>& tab);
+cudaError_t load_colops(const ColSpec* specs, int n, const std::vector<double>& tab, double* dev, cudaStream_t st);
+cudaError_t make_colops(ColSpec* specs, int n, cudaStream_t st);   // both, in memory freed with the first
 void free_colop(DevColOp& d);
 // Right-hand side weights for an output scaled by `scale`.
 ColWeights col_weights(const DevColOp& d, double scale);

@@ -324,7 +324,7 @@ int col_rows_per_chunk(int nsys, int dir) {
 
 // The column solve's view of the system with `pad` identity rows before and after it (pad > 0
 // embeds an operator in the chunks of one with a longer system).
-// The host side of make_colop: everything but the device copy of the table `t`.
+// Everything but the device copy of the table `t`.
 static cudaError_t fill_colop(const HostOp& h, int S, int pad, DevColOp& out, std::vector<double>& t) {
   const int n0 = h.nsys(), nsys = n0 + 2 * pad;
   if (S < 1 || S > COL_MAXS || nsys < 2 * S) return cudaErrorInvalidValue;
@@ -380,27 +380,36 @@ static cudaError_t fill_colop(const HostOp& h, int S, int pad, DevColOp& out, st
   return cudaSuccess;
 }
 
-// Column operators share one device table, owned by the first of them.
-cudaError_t make_colops(const ColSpec* specs, int n, cudaStream_t st) {
-  std::vector<double> all;
-  std::vector<size_t> at(n);
+// Column operators share one device table: theirs one after the other in `tab`.
+cudaError_t fill_colops(ColSpec* specs, int n, std::vector<double>& tab) {
+  tab.clear();
   for (int i = 0; i < n; ++i) {
     std::vector<double> t;
     const cudaError_t e = fill_colop(*specs[i].h, specs[i].S, specs[i].pad, *specs[i].out, t);
     if (e != cudaSuccess) return e;
-    at[i] = all.size();
-    all.insert(all.end(), t.begin(), t.end());
-    all.resize((all.size() + 1) / 2 * 2);   // 16-byte rows
+    specs[i].at = tab.size();
+    tab.insert(tab.end(), t.begin(), t.end());
+    tab.resize((tab.size() + 1) / 2 * 2);   // 16-byte rows
   }
-  if (all.empty()) return cudaSuccess;      // explicit operators have no table
-  DevColOp& own = *specs[0].out;
-  cudaError_t e = cudaMalloc(&own.dtab, all.size() * sizeof(double));
-  if (e != cudaSuccess) return e;
-  // on the context's stream: a copy on the legacy stream would wait for the caller's work there
-  e = cudaMemcpyAsync(own.dtab, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+  return cudaSuccess;
+}
+
+cudaError_t load_colops(const ColSpec* specs, int n, const std::vector<double>& tab, double* dev, cudaStream_t st) {
+  // st holds nothing else: on the context's stream this would wait for all work queued there, on the
+  // legacy stream for the caller's
+  cudaError_t e = cudaMemcpyAsync(dev, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  for (int i = 0; i < n; ++i) specs[i].out->op.tab = own.dtab + at[i];
+  for (int i = 0; i < n; ++i) specs[i].out->op.tab = dev + specs[i].at;
   return e;
+}
+
+cudaError_t make_colops(ColSpec* specs, int n, cudaStream_t st) {
+  std::vector<double> tab;
+  cudaError_t e = fill_colops(specs, n, tab);
+  if (e != cudaSuccess || tab.empty()) return e;   // explicit operators have no table
+  DevColOp& own = *specs[0].out;
+  if ((e = cudaMalloc(&own.dtab, tab.size() * sizeof(double))) != cudaSuccess) return e;
+  return load_colops(specs, n, tab, own.dtab, st);
 }
 
 ColWeights col_weights(const DevColOp& d, double scale) {

@@ -49,21 +49,18 @@ cudaError_t launch_dir(int pass, const ColArgs& a, const ColDir& d, int LW, int 
 
 int col_lines(const ColDir& d) { return lines_per_cta(d.d.op.nch); }
 
-cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out, RowOps& rows, cudaStream_t st) {
-  ColSpec specs[6];
-  int n = 4;
-  rows.c = row_c_shape(hd[0].nsys());
-  if (rows.c.S) specs[n++] = ColSpec{&hd[0], rows.c.S, 0, &rows.d};
-  if (const int S = row_f_rows(hf[0].nsys())) specs[n++] = ColSpec{&hf[0], S, 0, &rows.f};
+cudaError_t fill_coldirs(const HostOp* hd, const HostOp* hf, ColDir* out, RowOps& rows, std::vector<ColSpec>& specs,
+                         std::vector<double>& tab) {
   for (int d = 1; d < 3; ++d) {
     const int S = col_rows_per_chunk(hf[d].nsys(), d);
-    specs[2 * d - 2] = ColSpec{&hd[d], S, (hf[d].nsys() - hd[d].nsys()) / 2, &out[d].d};
-    specs[2 * d - 1] = ColSpec{&hf[d], S, 0, &out[d].f};
+    specs.push_back({&hd[d], S, (hf[d].nsys() - hd[d].nsys()) / 2, &out[d].d});
+    specs.push_back({&hf[d], S, 0, &out[d].f});
   }
-  return make_colops(specs, n, st);
+  rows.c = row_c_shape(hd[0].nsys());
+  if (rows.c.S) specs.push_back({&hd[0], rows.c.S, 0, &rows.d});
+  if (const int S = row_f_rows(hf[0].nsys())) specs.push_back({&hf[0], S, 0, &rows.f});
+  return fill_colops(specs.data(), (int)specs.size(), tab);
 }
-
-void free_coldirs(ColDir* dirs) { free_colop(dirs[1].d); }
 
 cudaError_t launch_col_pass(int pass, const PassArgs& p, const double* G, const ColDir& d, cudaStream_t st) {
   ColArgs a{};

@@ -22,9 +22,10 @@ int row_c_tiles(const BoxGeo& g, const RowOps& r);   // CTAs of pass C, one part
 cudaError_t launch_row_c(const PassArgs& p, const RowOps& r, cudaStream_t st);
 cudaError_t launch_row_filter(const PassArgs& p, const RowOps& r, cudaStream_t st);
 
-// Directions 1 and 2 of cols[3] and the x operators, from the operators of the three directions.
-cudaError_t make_coldirs(const HostOp* hd, const HostOp* hf, ColDir* cols, RowOps& rows, cudaStream_t st);
-void free_coldirs(ColDir* dirs);
+// Directions 1 and 2 of cols[3] and the x operators, from the operators of the three directions: all but
+// the device copy of their table (load_colops).
+cudaError_t fill_coldirs(const HostOp* hd, const HostOp* hf, ColDir* cols, RowOps& rows, std::vector<ColSpec>& specs,
+                         std::vector<double>& tab);
 int col_lines(const ColDir& d);   // lines per CTA
 // pass: ColPass of tgv_cols.cuh (0 filter in place, 1 gradients, 2 R += D(G), 3 update and filter);
 // G: the fields that passes 1 to 3 differentiate.

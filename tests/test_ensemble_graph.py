@@ -73,3 +73,22 @@ def test_shapes_changed_after_the_first_step(change):
         change(together[1])
     _equal(alone, together)
     ens.close()
+
+
+@pytest.mark.parametrize("own", [True, False])
+def test_creation_waits_for_no_queued_work(own):
+    """Boxes and schemes are made while the context's stream (own) or the legacy stream is busy."""
+    import torch
+    import astr_gpu_b200 as ag
+    side = torch.cuda.Stream()
+    ctx = ag.Context(0, stream=side)
+    make = lambda: (ag.TGVSolver(ctx, 24), ag.fd_scheme_initiate(ctx, "643c", 3, 48))  # noqa: E731
+    keep = [make()]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side if own else torch.cuda.default_stream()):
+        torch.cuda._sleep(1_000_000_000)   # about half a second
+        busy = torch.cuda.Event()
+        busy.record()
+    keep.append(make())
+    assert not busy.query()
+    torch.cuda.synchronize()
