@@ -1,5 +1,5 @@
 """The column solve of the line operators (csrc/colsolve.cuh): chunks of S rows per thread, the
-left-over slots in the middle chunk, carries combined over the chunks.
+left-over slots at the end of chunk 1, carries combined over the chunks.
 
 On the CPU: the algorithm restated in numpy against the reference's sequential Thomas sweep
 (commfunc.F90:790-813) on the oracle's factors. On the GPU: every operator at the sizes where the
@@ -23,79 +23,124 @@ def _thomas(ac, d):
     return y
 
 
-def _columns(ac, d, S):
-    a1, a2, a3 = (x.copy() for x in ac)
-    n = len(d)
-    a1[-1], a2[0], a3[0] = 0.0, 1.0, 0.0
+def _tables(ac, S, pad):
+    """fill_colop's chunk tables (schemes.cu): the system with `pad` identity rows before and after it,
+    the slots left over as the last ones of chunk 1, the chunks c_lo..nch-2 with one coefficient set,
+    and the converged ac2 (k2) taken out of every row's."""
+    n0 = len(ac[0])
+    n = n0 + 2 * pad
     nch = max(3, -(-n // S))
-    rag, nv = nch // 2, n - (nch - 1) * S
-    e1, e2, e3, v = -np.ones((nch, S)), np.zeros((nch, S)), -np.ones((nch, S)), np.zeros((nch, S))
+    nv = n - (nch - 1) * S
+    e1, e2, e3 = -np.ones((nch, S)), np.zeros((nch, S)), -np.ones((nch, S))
     for c in range(nch):
-        m = nv if c == rag else S
-        r = c * S - (S - nv if c > rag else 0)
-        e1[c, :m], e2[c, :m], e3[c, :m], v[c, :m] = a1[r:r + m], a2[r:r + m], a3[r:r + m], d[r:r + m]
+        for k in range(S):
+            r = c * S + k - (S - nv if c > 1 else 0) - pad
+            if c == 1 and k >= nv:
+                continue
+            if r < 0 or r >= n0:
+                e1[c, k], e2[c, k], e3[c, k] = 0.0, 1.0, 0.0
+            else:
+                e1[c, k] = 0.0 if r == n0 - 1 else ac[0][r]
+                e2[c, k], e3[c, k] = (1.0, 0.0) if r == 0 else (ac[1][r], ac[2][r])
+    tabs = np.stack([e1, e2, e3], axis=-1)
+    c_lo, k2 = nch - 1, 1.0
+    if nch > 3 and np.all(tabs[nch - 2] == tabs[nch - 2, 0]):
+        c_lo, k2 = nch - 2, e2[nch - 2, 0]
+        while c_lo > 2 and np.array_equal(tabs[c_lo - 1], tabs[nch - 2]):
+            c_lo -= 1
+        c_lo = min(c_lo + (c_lo % 2 == 0), nch - 1)
+    return e1, e2 / k2, e3, nch, nv, c_lo, k2
+
+
+def _columns(ac, d, S, pad=0):
+    """col_solve's sweeps (colsolve.cuh): converged chunks take no factor per row (the right-hand side
+    carries k2), table chunks the rest of ac2."""
+    e1, e2, e3, nch, nv, c_lo, k2 = _tables(ac, S, pad)
+    rows = np.concatenate([np.zeros(pad), d, np.zeros(pad)]) * k2
+    v = np.zeros((nch, S))
+    for c in range(nch):
+        m = nv if c == 1 else S
+        r = c * S - (S - nv if c > 1 else 0)
+        v[c, :m] = rows[r:r + m]
+    const = [c_lo <= c < nch - 1 for c in range(nch)]
+    last = nch - 2
+    pf, qb = np.cumprod(-e3, axis=1), np.cumprod((-e1)[:, ::-1], axis=1)[:, ::-1]
+    k1, k3 = e1[last, 0], e3[last, 0]
     G, B = np.zeros(nch), np.zeros(nch)
     for c in range(nch):
         g = 0.0
         for t in range(S):
-            g = v[c, t] * e2[c, t] - g * e3[c, t]
+            g = v[c, t] - k3 * g if const[c] else v[c, t] * e2[c, t] - e3[c, t] * g
             v[c, t] = g
         G[c] = g
     for c in range(nch):
         cin = 0.0
         for j in range(c):
-            cin = np.prod(-e3[j]) * cin + G[j]
-        y = np.cumprod(-e3[c]) * cin + v[c]
-        if c == rag:
+            cin = (pf[j, -1] if j < c_lo else pf[last, -1]) * cin + G[j]
+        y = (pf[last] if const[c] else pf[c]) * cin + v[c]
+        if c == 1:
             y[nv:] = 0.0
         g = 0.0
         for t in range(S - 1, -1, -1):
-            g = y[t] - e1[c, t] * g
+            g = y[t] - (k1 if const[c] else e1[c, t]) * g
             v[c, t] = g
         B[c] = g
-    for c in range(nch):
-        cb = 0.0
-        for j in range(nch - 1, c, -1):
-            cb = np.prod(-e1[j]) * cb + B[j]
-        v[c] += np.cumprod((-e1[c])[::-1])[::-1] * cb
-    return np.concatenate([v[c, :nv if c == rag else S] for c in range(nch)])
+    for c in range(nch - 1):
+        cb = B[nch - 1]
+        for j in range(nch - 2, c, -1):
+            cb = (qb[last, 0] if j >= c_lo else qb[j, 0]) * cb + B[j]
+        v[c] += (qb[last] if const[c] else qb[c]) * cb
+    x = np.concatenate([v[c, :nv if c == 1 else S] for c in range(nch)])
+    return x[pad:len(x) - pad]
 
 
+# S as col_rows_per_chunk picks it, and 25 as pass C has it; 263 and 1049 leave no slot over
 @pytest.mark.parametrize("dim,S", [(16, 5), (20, 9), (32, 9), (38, 9), (39, 17), (85, 17), (131, 33), (257, 33), (258, 33),
-                                   (1040, 33), (1060, 37)])
-@pytest.mark.parametrize("kind", ["deriv", "filter"])
+                                   (263, 33), (600, 25), (1040, 33), (1049, 33), (1060, 37)])
+@pytest.mark.parametrize("kind", ["deriv", "filter", "slow filter", "flux"])
 @pytest.mark.parametrize("ntype", [1, 2, 3, 4])
-def test_chunks_equal_thomas(kind, ntype, dim, S):
+@pytest.mark.parametrize("pad", [0, 2])
+def test_chunks_equal_thomas(kind, ntype, dim, S, pad):
     sch = {"deriv": lambda: oracle.fd_scheme_initiate("643c", ntype, dim),
-           "filter": lambda: oracle.compact_filter_initiate(ntype, dim, 0.49, 1.11, 0.98)}[kind]()
+           "filter": lambda: oracle.compact_filter_initiate(ntype, dim, 0.49, 1.11, 0.98),
+           # factors that go on changing along the line: no converged chunks
+           "slow filter": lambda: oracle.compact_filter_initiate(ntype, dim, 0.5, 1.11, 0.98),
+           "flux": lambda: oracle.compact_flux_initiate(ntype, dim, "-", 0.3)}[kind]()
     ac = sch.ac()[2:]
+    if len(ac[0]) + 2 * pad < 2 * S:
+        pytest.skip("fewer than two chunks of rows")
     d = np.random.default_rng(dim).standard_normal(len(ac[0]))
-    ref, got = _thomas(ac, d), _columns(ac, d, S)
-    # both orders round each row a few times; errors decay along the line with the factors
-    assert np.abs(got - ref).max() <= 40 * np.finfo(float).eps * np.abs(ref).max()
+    ref, got = _thomas(ac, d), _columns(ac, d, S, pad)
+    # both orders round each row a few times; errors decay along the line with the factors, or at
+    # alpha = 0.5 add up over it
+    eps = 40 * (dim if kind == "slow filter" else 1) * np.finfo(float).eps
+    assert np.abs(got - ref).max() <= eps * np.abs(ref).max()
+    if dim >= 600:   # the sizes that exercise converged chunks do have them
+        nch, _, c_lo = _tables(ac, S, pad)[3:6]
+        assert (c_lo < nch - 1) == (kind != "slow filter")
 
 
 def _rel(a, b):
     return np.abs(a - b).max() / max(np.abs(b).max(), 1e-300)
 
 
-def _apply(ag, ctx, kind, ntype, dim, f, d, lb, **kw):
+def _apply(ag, ctx, kind, ntype, dim, f, d, lb, wind="+", alfa=0.49, **kw):
     if kind == "deriv":
         return ag.central(ctx, ag.fd_scheme_initiate(ctx, "643c", ntype, dim), f, d, lbound=lb, **kw)
     if kind == "explicit":
         return ag.central(ctx, ag.fd_scheme_initiate(ctx, "643e", ntype, dim), f, d, lbound=lb, **kw)
     if kind == "filter":
-        return ag.compact_filter(ctx, ag.compact_filter_initiate(ctx, ntype, dim, 0.49, 1.11, 0.98), f, d, lbound=lb, **kw)
-    sch = ag.compact_flux_initiate(ctx, ntype, dim, "+", 0.3)
+        return ag.compact_filter(ctx, ag.compact_filter_initiate(ctx, ntype, dim, alfa, 1.11, 0.98), f, d, lbound=lb, **kw)
+    sch = ag.compact_flux_initiate(ctx, ntype, dim, wind, 0.3)
     return (ag.flux_compact if kind == "flux" else ag.flux_difference)(ctx, sch, f, d, lbound=lb, **kw)
 
 
-def _oracle(kind, ntype, dim, f, d, lb):
+def _oracle(kind, ntype, dim, f, d, lb, wind="+", alfa=0.49):
     if kind in ("deriv", "explicit"):
         return oracle.fd_scheme_initiate("643c" if kind == "deriv" else "643e", ntype, dim).apply3d(f, d, lbound=lb)
     if kind == "filter":
-        return oracle.compact_filter_initiate(ntype, dim, 0.49, 1.11, 0.98).apply3d(f, d, lbound=lb)
-    fh = oracle.compact_flux_initiate(ntype, dim, "+", 0.3).apply3d(f, d, lbound=lb)
+        return oracle.compact_filter_initiate(ntype, dim, alfa, 1.11, 0.98).apply3d(f, d, lbound=lb)
+    fh = oracle.compact_flux_initiate(ntype, dim, wind, 0.3).apply3d(f, d, lbound=lb)
     if kind == "flux":
         return fh
     n = fh.shape[d]
@@ -106,6 +151,14 @@ def _oracle(kind, ntype, dim, f, d, lb):
 def ctx():
     import astr_gpu_b200 as ag
     return ag.Context(0)
+
+
+def _lines(dim, d, rng):
+    shape, lb = [35, 34, 3], [0, 0, 0]   # other extents past one tile of 32 lines
+    if d == 2:
+        shape = [35, 3, 3]
+    shape[d], lb[d] = dim + 1 + 2 * HM, -HM
+    return np.asfortranarray(rng.standard_normal(shape)), lb
 
 
 # around every change of the rows per chunk (systems of 15, 18, 46, 91, 177, 1057 rows), of the lines
@@ -122,12 +175,59 @@ def test_sizes(ctx, kind, ntype, dim):
         pytest.skip("the filter needs 16 nodes")
     rng = np.random.default_rng(dim)
     for d in range(3):
-        shape, lb = [35, 34, 3], [0, 0, 0]   # other extents past one tile of 32 lines
-        if d == 2:
-            shape = [35, 3, 3]
-        shape[d], lb[d] = dim + 1 + 2 * HM, -HM
-        f = np.asfortranarray(rng.standard_normal(shape))
+        f, lb = _lines(dim, d, rng)
         assert _rel(_apply(ag, ctx, kind, ntype, dim, f, d, lb), _oracle(kind, ntype, dim, f, d, lb)) <= 1e-12
+
+
+# one physical end, and the downwind flux, at the same edges
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [16, 17, 39, 90, 176, 263, 1050])
+@pytest.mark.parametrize("kind,wind", [("deriv", "+"), ("explicit", "+"), ("filter", "+"), ("flux", "-"), ("fluxdiff", "-")])
+@pytest.mark.parametrize("ntype", [1, 2, 3])
+def test_one_physical_end(ctx, kind, wind, ntype, dim):
+    import astr_gpu_b200 as ag
+    for d in range(3):
+        f, lb = _lines(dim, d, np.random.default_rng(dim))
+        ref = _oracle(kind, ntype, dim, f, d, lb, wind)
+        assert _rel(_apply(ag, ctx, kind, ntype, dim, f, d, lb, wind), ref) <= 1e-12
+
+
+# alpha = 0.5: factors that never converge, every chunk reads its own. The system's condition grows with
+# the square of its length, and with it what rounding the right-hand side and each sweep may change
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [17, 39, 90, 176, 263, 1050])
+@pytest.mark.parametrize("ntype", [3, 4])
+def test_filter_without_converged_factors(ctx, ntype, dim):
+    import astr_gpu_b200 as ag
+    a1, a2, a3 = oracle.compact_filter_initiate(ntype, dim, 0.5, 1.11, 0.98).ac()[2:]
+    lower, upper = a3[1:] / a2[1:], a1[:-1] / np.concatenate([[1.0], a2[1:-1]])
+    A = np.eye(len(a1)) + np.diag(lower, -1) + np.diag(upper, 1)
+    tol = 16 * np.finfo(float).eps * np.linalg.cond(A, np.inf)
+    assert tol <= 1e-7
+    for d in range(3):
+        f, lb = _lines(dim, d, np.random.default_rng(dim))
+        assert _rel(_apply(ag, ctx, "filter", ntype, dim, f, d, lb, alfa=0.5),
+                    _oracle("filter", ntype, dim, f, d, lb, alfa=0.5)) <= max(tol, 1e-12)
+
+
+# a line that holds a NaN or an infinity leaves the lines beside it as they are, bit for bit
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("dim", [39, 176, 300])
+@pytest.mark.parametrize("kind", ["deriv", "filter", "flux"])
+def test_bad_line_stays_alone(ctx, kind, dim, bad):
+    import astr_gpu_b200 as ag
+    for d in range(3):
+        f, lb = _lines(dim, d, np.random.default_rng(dim))
+        ref = _apply(ag, ctx, kind, 3, dim, f, d, lb)
+        at = [2, 2, 2]
+        at[d] = HM + dim // 2
+        f[tuple(at)] = bad
+        got = _apply(ag, ctx, kind, 3, dim, f, d, lb)
+        at[d] = slice(None)
+        assert not np.isfinite(got[tuple(at)]).all()
+        got[tuple(at)] = ref[tuple(at)] = 0.0
+        np.testing.assert_array_equal(got, ref)
 
 
 # x extents at the edges of flattened and per-row tiles (16 and 32 lines)
