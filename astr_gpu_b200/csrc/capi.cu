@@ -255,6 +255,13 @@ std::pair<DevOp, DevOp>& get_ops(astr_state* st, int dir, int S, int WPL) {
   return st->ops.emplace(key, o).first->second;
 }
 
+// Tables of the passes on lane-scan kernels, before a capture: their blocking copies fail in the capture of
+// a stream that synchronises with the legacy stream.
+void make_lane_tables(astr_state* st) {
+  for (int id = 0; id < NCFG; ++id)
+    if (!st->use_col[id]) get_ops(st, CFG_DIR[id], st->cfg[id].S, st->cfg[id].WPL);
+}
+
 // Number of pass-C CTAs, i.e. of partial sums the diagnostics reduce.
 int diag_parts(astr_state* st) {
   if (st->use_col[CFG_C]) return row_c_tiles(st->g, st->rows);
@@ -1070,6 +1077,7 @@ int astr_rk3_step(astr_state* st, double dt, int nsteps) {
     if (st->use_graph) {
       if (!st->gexec[variant] || st->gdt[variant] != dt) {
         if (st->gexec[variant]) { cudaGraphExecDestroy(st->gexec[variant]); st->gexec[variant] = nullptr; }
+        make_lane_tables(st);
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
         cudaError_t e = run_step(st, dt, variant == 1);
@@ -1220,6 +1228,7 @@ int ens_capture(astr_ensemble* e, int variant) {
   std::vector<int> order(nbox);
   for (int b = 0; b < nbox; ++b) order[b] = b;
   std::sort(order.begin(), order.end(), [&](int x, int y) { return box_nodes(e->boxes[x]) > box_nodes(e->boxes[y]); });
+  for (astr_state* st : e->boxes) make_lane_tables(st);
   std::vector<int64_t> load(nbr, 0);
   std::vector<cudaStream_t> strm(nbr, nullptr);
   std::vector<cudaEvent_t> ev(nbr + 1, nullptr);

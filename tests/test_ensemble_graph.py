@@ -92,3 +92,29 @@ def test_creation_waits_for_no_queued_work(own):
     keep.append(make())
     assert not busy.query()
     torch.cuda.synchronize()
+
+
+def test_lane_scan_box_on_a_blocking_stream():
+    """A stream that synchronises with the legacy stream: the tables of a box's lane-scan kernels are
+    made before the step is captured."""
+    import ctypes
+    import torch
+    import astr_gpu_b200 as ag
+    torch.zeros(1, device="cuda")
+    raw = ctypes.c_void_p()
+    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(raw))) == 0
+    ctx = ag.Context(0, stream=raw.value)
+    sizes = [24, 16]
+    alone, together = _boxes(ctx, sizes, 1), _boxes(ctx, sizes, 1)
+    dt = np.array([0.05 / n for n in sizes])
+    ens = ag.Ensemble(ctx, together)
+    ens.step(dt, 2)
+    for s, d in zip(alone, dt):
+        s.rk3(d, 2)
+    _equal(alone, together)
+    ens.close()
+    for s in alone + together:
+        s.close()
+    ctx.synchronize()
+    ctx.close()
+    torch.cuda.cudart().cudaStreamDestroy(raw.value)
