@@ -510,13 +510,7 @@ cudaError_t autotune(astr_state* st) {
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
-  // pass A is timed without and with the owed filter along A fused in; the filter goes into its
-  // own pass F_A only where A + F_A beat the fused pass
-  const bool filt = st->p.filter_on != 0;
-  float tbest[NCFG], tfused = 1e30f;
-  PassCfg fusedc = st->cfg[CFG_A];
   for (int id = 0; id < NCFG; ++id) {
-    tbest[id] = 0.0f;
     if (st->use_col[id]) continue;
     const int dir = CFG_DIR[id], pass = CFG_PASS[id];
     const int nsys = st->hf[dir].nsys();
@@ -547,41 +541,32 @@ cudaError_t autotune(astr_state* st) {
         c.S = L.S; c.WPL = L.WPL; c.TI = ti; c.LP = tile_pitch(dim, ti, L.S); c.LPW = sh.lpw; c.FPS = sh.fps;
         const PassCfg saved = st->cfg[id];
         st->cfg[id] = c;
-        for (int fused = 0; fused < ((id == CFG_A && filt) ? 2 : 1); ++fused) {
-          PassArgs a = base_args(st, id);
-          a.q = st->Q1; a.D = st->DA; a.DA = st->DA; a.DB = st->DB;
-          // stage 2-3 form of the update, reading q (the scratch copy) and qsave (the live state,
-          // only read) from distinct arrays as the step does; values stay bounded: q <- (q + q) / 2
-          a.qsave = st->Q0; a.qout = st->Q1; a.mode = 1; a.do_filter = (id == CFG_A) ? fused : st->p.filter_on;
-          a.c1 = 0.5; a.c2 = 0.5; a.c3 = 0.0; a.dt = 0.0;
-          float ms = 1e30f;
-          if ((e = launch_pass(pass, a, c.S, c.WPL, sm)) == cudaSuccess) {
-            cudaEventRecord(t0, sm);
-            for (int r = 0; r < 4 && e == cudaSuccess; ++r) e = launch_pass(pass, a, c.S, c.WPL, sm);
-            cudaEventRecord(t1, sm);
-            cudaEventSynchronize(t1);
-            cudaEventElapsedTime(&ms, t0, t1);
-          }
-          if (e != cudaSuccess) {   // a shape the device cannot launch (e.g. too much shared memory)
-            cudaGetLastError();
-            e = cudaSuccess;
-            ms = 1e30f;
-          }
-          if (fused) {
-            if (ms < tfused) { tfused = ms; fusedc = c; }
-          } else if (ms < best) {
-            best = ms; bestc = c;
-          }
+        PassArgs a = base_args(st, id);
+        a.q = st->Q1; a.D = st->DA; a.DA = st->DA; a.DB = st->DB;
+        // stage 2-3 form of the update, reading q (the scratch copy) and qsave (the live state,
+        // only read) from distinct arrays as the step does; values stay bounded: q <- (q + q) / 2
+        a.qsave = st->Q0; a.qout = st->Q1; a.mode = 1;
+        // pass A in the form the step runs: with the owed filter along A fused in, or without
+        a.do_filter = st->p.filter_on && !(id == CFG_A && st->split_fa);
+        a.c1 = 0.5; a.c2 = 0.5; a.c3 = 0.0; a.dt = 0.0;
+        float ms = 1e30f;
+        if ((e = launch_pass(pass, a, c.S, c.WPL, sm)) == cudaSuccess) {
+          cudaEventRecord(t0, sm);
+          for (int r = 0; r < 4 && e == cudaSuccess; ++r) e = launch_pass(pass, a, c.S, c.WPL, sm);
+          cudaEventRecord(t1, sm);
+          cudaEventSynchronize(t1);
+          cudaEventElapsedTime(&ms, t0, t1);
+        }
+        if (e != cudaSuccess) {   // a shape the device cannot launch (e.g. too much shared memory)
+          cudaGetLastError();
+          e = cudaSuccess;
+          ms = 1e30f;
         }
         st->cfg[id] = saved;
+        if (ms < best) { best = ms; bestc = c; }
       }
     }
     st->cfg[id] = bestc;
-    tbest[id] = best;
-  }
-  if (!st->use_col[CFG_A]) {
-    st->split_fa = filt && tbest[CFG_A] + tbest[CFG_FA] < tfused;
-    if (filt && !st->split_fa) st->cfg[CFG_A] = fusedc;
   }
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);

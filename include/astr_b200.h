@@ -176,8 +176,10 @@ int astr_state_use_graph(astr_state* st, int on);
 int astr_state_split_filter(astr_state* st, int on);
 /* Per-pass autotuning of the launch shape (rows per lane, warps per line, lines per CTA) at the
  * first RK3 step of a state, on scratch copies of the live fields (default on above 100^3 nodes),
- * for the passes that run a lane-scan kernel: C and filter-C; the y and z passes run column solves
- * whose shape follows from the box. */
+ * for the passes that run a lane-scan kernel: pass C of boxes of more than 822 intervals along x,
+ * filter-C of more than 1049, and pinned passes when the call comes after the pin. All others run
+ * column solves, whose shape follows from the box; pass A is tuned in the form that
+ * astr_state_split_filter set. */
 int astr_state_autotune(astr_state* st, int on);
 /* Launch shape of each pass A, B, C, A', B', filter-C, filter-A as (S, WPL, TI, LP, LPW, FPS):
  * 42 ints. A pass that runs as a column solve reports its rows per chunk S, WPL 0 and its lines per

@@ -93,3 +93,19 @@ def test_reported_shapes(ctx):
     s.set_launch_shape("B", 9, 2, 8)
     assert s.launch_shapes()["B"][:3] == (9, 2, 8)
     s.close()
+
+
+def test_tuning_leaves_the_filter_where_the_caller_put_it(ctx):
+    """split_filter(False), then autotune(True): the tuned step still applies the filter along y in
+    pass A (the timings then hold no launch of it as a pass of its own)."""
+    import ctypes
+    import astr_gpu_b200 as ag
+    s = ag.TGVSolver(ctx, 40, 64, 32)   # 71 rows along y: the smallest layout is a candidate
+    s.split_filter(False)
+    s.autotune(True)
+    s.init_tgv()
+    s.rk3(1e-3, 2)
+    ms = (ctypes.c_double * 8)()
+    ctx.check(ctx.L.astr_pass_timings(s._h, 1e-3, 1, ms))
+    assert ms[0] > 0.0 and ms[7] == 0.0
+    s.close()
