@@ -8,6 +8,7 @@
 //    lines are contiguous in x) and walk the nodes with stride 32*WPL. Each thread keeps one
 //    line in this role, so no index arithmetic beyond one multiply-add per node.
 #pragma once
+#include "bulkcopy.cuh"
 #include "tgv.cuh"
 
 namespace astr {
@@ -144,37 +145,6 @@ __device__ __forceinline__ void load_tile(const TileCtx<DIR, WPL, LW>& c, double
   for (; n <= dim + HT; n += nst) cp_async8(trow + n, src + (int64_t)(n - dim) * sd);
 }
 
-// ---- bulk copies completing on an mbarrier (the copy engine moves whole contiguous rows)
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-// Poll the barrier's phase `parity` at most `limit` times; false when it did not complete.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int limit) {
-  for (int it = 0; it < limit; ++it) {
-    unsigned done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done)
-                 : "r"(smem_u32(bar)), "r"(parity)
-                 : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-constexpr int kBarrierPolls = 1 << 22;   // bounded wait (far beyond any copy's duration)
-
 // Stage `nf` fields of the x lines of a tile with one bulk copy per line and field (nodes 0..dim
 // are contiguous: one row of the padded box, 16-byte aligned), completing on one mbarrier; then
 // the periodic halos -HT..-1 and dim+1..dim+HT are filled from the staged rows in shared memory.
@@ -200,7 +170,7 @@ __device__ __forceinline__ void stage_x_bulk(const TileCtx<0, WPL>& c, double* T
   if (!c.svalid) {
     for (int m = 0; m < nf; ++m) c.for_nodes(-HT, dim + HT, [&](int o, int) { T[m * tsz + o] = 1.0; });
   }
-  if (!mbar_wait(bar, 0, kBarrierPolls) && threadIdx.x == 0) atomicOr(a.err, 2);
+  mbar_wait_or_flag(bar, a.err);
   if (c.svalid) {
     for (int m = 0; m < nf; ++m) {
       double* row = T + m * tsz + c.sl * c.LP + HT;

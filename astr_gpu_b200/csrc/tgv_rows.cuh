@@ -17,6 +17,7 @@
 // 8 lines in the filter) the pitch is 2 mod 16 doubles, so eight systems hit the even bank pairs and
 // the next chunk, an odd number of rows away, the odd ones; with NL = 4 and 8 it is 1 mod 16.
 #pragma once
+#include "bulkcopy.cuh"
 #include "tgv.cuh"
 
 namespace astr {
@@ -42,36 +43,6 @@ struct RowArgs {
 };
 
 namespace row_detail {
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bar_init(uint64_t* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* bar, unsigned bytes) {
-  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void row_copy(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-// Wait for the barrier's first phase, at most `limit` polls.
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, int limit) {
-  for (int it = 0; it < limit; ++it) {
-    unsigned done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done)
-                 : "r"(smem_addr(bar))
-                 : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-constexpr int kPolls = 1 << 22;   // far beyond any copy's duration
 
 __device__ __forceinline__ double viscosity(const Thermo& th, double t) { return t * sqrt(t) * th.tc1 / (t + th.tc); }
 
@@ -149,14 +120,14 @@ __global__ void __launch_bounds__(256, 2) k_row_c(const __grid_constant__ RowArg
   const int nl = min(NL, a.g.N[1] + 1 - y0);
   const int64_t fs = a.g.fs, row0 = (int64_t)y0 * a.g.st[1] + (int64_t)z * a.g.st[2];
   const unsigned bytes = (unsigned)(((dim + 1) * 8 + 15) & ~15);   // within the padded row
-  if (threadIdx.x == 0) bar_init(&bar);
+  if (threadIdx.x == 0) mbar_init(&bar, 1);
   __syncthreads();
-  if (threadIdx.x == 0) bar_expect(&bar, bytes * 5u * (unsigned)nl);
+  if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, bytes * 5u * (unsigned)nl);
   if (threadIdx.x < 32) {
     __syncwarp();
     for (int r = threadIdx.x; r < 5 * nl; r += 32) {
       const int m = r / nl, l = r - m * nl;
-      row_copy(T + (m * NL + l) * LT, a.q + m * fs + row0 + l * a.g.st[1], bytes, &bar);
+      bulk_g2s(T + (m * NL + l) * LT, a.q + m * fs + row0 + l * a.g.st[1], bytes, &bar);
     }
   } else if (threadIdx.x < 32 + 8 * NL) {   // the gradients along y and z start moving into L2
     const int r = threadIdx.x - 32, m = r / NL, l = r - m * NL;
@@ -168,7 +139,7 @@ __global__ void __launch_bounds__(256, 2) k_row_c(const __grid_constant__ RowArg
   if (nl < NL)   // lines past the box: finite filler for the solves, never stored
     for (int r = threadIdx.x; r < 5 * NL * LG; r += NT)
       if ((r / LG) % NL >= nl) G[r] = 0.0;
-  if (!bar_wait(&bar, kPolls) && threadIdx.x == 0) atomicOr(a.err, 2);
+  mbar_wait_or_flag(&bar, a.err);
   const int l = threadIdx.x / TPL, j0 = threadIdx.x % TPL;
   const bool on = l < nl;
   double* Tl = T + l * LT;
@@ -299,17 +270,17 @@ __global__ void __launch_bounds__(256, 2) k_row_filter(const __grid_constant__ R
   const int nl = min(LW, a.g.N[1] + 1 - y0);
   double* f = a.q + m * a.g.fs + (int64_t)y0 * a.g.st[1] + (int64_t)z * a.g.st[2];
   const unsigned bytes = (unsigned)(((dim + 1) * 8 + 15) & ~15);
-  if (threadIdx.x == 0) bar_init(&bar);
+  if (threadIdx.x == 0) mbar_init(&bar, 1);
   __syncthreads();
-  if (threadIdx.x == 0) bar_expect(&bar, bytes * (unsigned)nl);
+  if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, bytes * (unsigned)nl);
   if (threadIdx.x < 32) {
     __syncwarp();
-    if (threadIdx.x < nl) row_copy(G + threadIdx.x * LG + ROW_HF, f + threadIdx.x * a.g.st[1], bytes, &bar);
+    if (threadIdx.x < nl) bulk_g2s(G + threadIdx.x * LG + ROW_HF, f + threadIdx.x * a.g.st[1], bytes, &bar);
   }
   const int l = threadIdx.x % LW, p = threadIdx.x / LW, c = col_chunk(a.op, p);
   const bool act = p < nch;
   double* line = G + l * LG + ROW_HF;
-  if (!bar_wait(&bar, kPolls) && threadIdx.x == 0) atomicOr(a.err, 2);
+  mbar_wait_or_flag(&bar, a.err);
   const int n0 = col_node<S>(a.op, c);
   double v[S];
   if (act) {
@@ -335,7 +306,7 @@ __global__ void __launch_bounds__(256, 2) k_row_filter(const __grid_constant__ R
   __syncthreads();
   if (threadIdx.x < nl) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(f + threadIdx.x * a.g.st[1]),
-                 "r"(smem_addr(G + threadIdx.x * LG + ROW_HF)), "r"(bytes)
+                 "r"(smem_u32(G + threadIdx.x * LG + ROW_HF)), "r"(bytes)
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
