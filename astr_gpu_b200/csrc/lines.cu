@@ -10,8 +10,9 @@
 // y and z lines: the LW lines are adjacent in x, so each row is one piece of LW * 8 bytes that goes
 // from HBM into the registers of LW threads; nothing is staged. x lines: the lines are copied to a
 // shared-memory tile with asynchronous copies (node-fastest), each thread reads its chunk's window
-// from its line (the pitch is odd, so the 16 lines of a half warp hit different banks), and results
-// go back through the tile for coalesced stores.
+// from its line, and results go back through the tile for coalesced stores. 16 lines with an odd
+// pitch, or from 33 rows per chunk on 8 lines with a pitch of 2 mod 16: either way a half warp hits
+// 16 different bank pairs.
 #include "internal.h"
 
 namespace astr {
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(S >= 17 ? 512 : 256, S >= 17 ? 1 : 2)
   }
 }
 
-// x lines, through a tile of LW lines with nodes -HL..dim+HL (pitch LP, odd).
+// x lines, through a tile of LW lines with nodes -HL..dim+HL (pitch LP).
 template <int S, int KIND, int LW>
 __global__ void __launch_bounds__(S >= 17 ? 512 : 320, S >= 17 ? 1 : 2)
     k_line_row(LineOp op, ColOp co, ColConst<S> k, LineArgs a, int LP) {
@@ -283,7 +284,9 @@ template <int S, int KIND>
 static cudaError_t launch_sk(const DevColOp& op, const LineArgs& a, int nfields, cudaStream_t st) {
   if (a.dir != 0) {
     // 32 lines per CTA up to eight chunks, 16 beyond: two CTAs of 128 registers fit on an SM
-    if (op.op.nch <= 8) return launch_col<S, KIND, 32>(op, a, nfields, st);
+    if constexpr (S < 37) {   // 37 rows: 29 chunks or more
+      if (op.op.nch <= 8) return launch_col<S, KIND, 32>(op, a, nfields, st);
+    }
     if constexpr (S >= 33) return launch_col<S, KIND, 16>(op, a, nfields, st);
     return cudaErrorInvalidValue;
   }
