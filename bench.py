@@ -32,16 +32,16 @@ sys.path.insert(0, ROOT)
 
 METRIC = "RK3 grid-point updates/s FP64 TGV 512³ + %HBM peak; adjoint:forward step time"
 UNIT = "grid-point RK3 updates/s"
-B_ALG_STEP = 2504.0      # algorithmic bytes per unique grid point per RK3 step (pass model)
-B_ALG_STEP_FUSED = 2384.0   # the same with the owed filter along A fused into pass A
 # fields read + written per stored point by one launch of each pass (B' reads q for the c2 term at
-# two of the three stages; A counts the primitives' 9 fields and its own 8, B 8; with the lane-scan
-# kernels pinned for pass A and the owed filter fused into it, A moves 14 fields)
+# two of the three stages; A counts the primitives' 9 fields and its own 8, B 8)
 PASS_NAMES = ["A", "B", "C", "A'", "B'", "F", "diag", "F_A"]   # astr_pass_timings order
 PASS_FIELDS = {"A": 17, "B": 8, "C": 28, "A'": 15, "B'": 20 + 10 / 3, "F": 10, "F_A": 10}
 PASS_PER_STEP = {"A": 3, "B": 3, "C": 3, "A'": 3, "B'": 3, "F": 3, "F_A": 3}
-# kernels of one filtered RK3 step in the timed region: 7 passes and the primitives per stage (6
-# passes with filter-A fused into the lane-scan pass A) and the diagnostics reduce
+# algorithmic bytes per unique grid point per RK3 step: 334 fields of 8 B
+B_ALG_STEP = 8.0 * sum(f * PASS_PER_STEP[k] for k, f in PASS_FIELDS.items())
+# kernels of one filtered RK3 step in the timed region: 7 passes and the primitives per stage, and the
+# diagnostics reduce
+LAUNCHES_PER_STEP = 3 * 8 + 1
 
 
 def peaks():
@@ -194,23 +194,20 @@ def run_ours(args, ws, rank, local):
     pk, pk_kind = peaks()
     pts = (n + 1) ** 3
     shares = {nm: per[i] * PASS_PER_STEP[nm] for i, nm in enumerate(PASS_NAMES) if nm in PASS_PER_STEP}
-    split_fa = per[PASS_NAMES.index("F_A")] > 0.0   # no F_A launches: filter-A fused into pass A
-    fields = dict(PASS_FIELDS, A=PASS_FIELDS["A"] if split_fa else 14)
     dom = max(shares, key=shares.get)
     di = PASS_NAMES.index(dom)
-    alg_bytes = fields[dom] * 8.0 * pts
+    alg_bytes = PASS_FIELDS[dom] * 8.0 * pts
     achieved = alg_bytes / (per[di] * 1e-3) / 1e9
     traffic = None
     tf = os.path.join(ROOT, "profiles", "dram_traffic.json")
     if os.path.exists(tf):
-        tkey = "A_fused" if dom == "A" and not split_fa else dom
-        traffic = json.load(open(tf)).get(str(n), {}).get(tkey)
+        traffic = json.load(open(tf)).get(str(n), {}).get(dom)
     roof = {"kernel": f"pass {dom}", "bound": "hbm", "achieved": achieved, "peak": pk, "unit": "GB/s",
             "frac": achieved / pk, "traffic": traffic, "peak_kind": pk_kind,
             "alg_bytes_per_launch": alg_bytes, "ms_per_launch": float(per[di]),
             "per_pass_ms": {nm: float(per[i]) for i, nm in enumerate(PASS_NAMES) if nm != "diag"},
             "diag_reduce_ms": float(per[6])}
-    step_bytes = (B_ALG_STEP if split_fa else B_ALG_STEP_FUSED) * n ** 3
+    step_bytes = B_ALG_STEP * n ** 3
     step_roof = {"bytes_per_step": step_bytes, "achieved": step_bytes / (ms_step * 1e-3) / 1e9, "peak": pk,
                  "unit": "GB/s", "frac": step_bytes / (ms_step * 1e-3) / 1e9 / pk, "peak_kind": pk_kind}
 
@@ -302,7 +299,7 @@ def run_ours(args, ws, rank, local):
                        "l2": "inputs larger than L2 (5 x 1.1 GB state per box)", "graph": "one CUDA graph per step",
                        "launch_shapes": shapes},
             "roofline": roof, "step_roofline": step_roof, "cpu_baseline": cpu, "e2e": e2e,
-            "gpu_launches": (3 * (8 if split_fa else 6) + 1) * args.steps, "clocks": clk.summary(),
+            "gpu_launches": LAUNCHES_PER_STEP * args.steps, "clocks": clk.summary(),
             "adjoint": adjoint, "ensemble": ensemble, "checkpoint": checkpoint,
         }
         print(json.dumps(line), flush=True)
@@ -332,7 +329,7 @@ def ensemble_boxes(ctx, specs):
 def measure_ensemble(ctx, stream, specs, steps, warmup, single, barrier=None):
     """Device time (CUDA events on the library's stream) of `steps` batched ensemble steps of the
     boxes `specs`, and, with `single`, of the same boxes stepped one at a time (each its own
-    autotuned shapes and per-step graph). Returns (ms batched, ms one at a time or None, boxes,
+    per-step graph). Returns (ms batched, ms one at a time or None, boxes,
     ensemble, time steps); the caller closes the boxes and the ensemble."""
     import torch
     import astr_gpu_b200 as ag
@@ -407,7 +404,7 @@ def run_ensemble(args, ws, rank, local):
     single = None
     if ms_solo is not None:
         single = {"value": pts_all * args.steps / (ms_solo * 1e-3), "ms_per_step": ms_solo / args.steps,
-                  "how": "each box alone, its own autotuned launch shapes and per-step CUDA graph, boxes in turn"}
+                  "how": "each box alone, its own per-step CUDA graph, boxes in turn"}
     e2e = None
     if not args.no_e2e:
         # end to end: upload every box's state from pinned host memory, step, download, per step
@@ -915,12 +912,15 @@ def run_checkpoint(args, ws, rank, local):
 
 def run_profile(args, local):
     """The workload for an ncu capture: `--steps` eager RK3 steps of a TGV box (no graph, no
-    timing, no JSON line), with the pass launch shapes pinned by `--shapes`."""
+    timing, no JSON line), with the passes that `--shapes` names pinned to their lane-scan kernels (an
+    entry as `launch_shapes` reports it; one of a column solve, 0 warps per line, is the default form)."""
     import astr_gpu_b200 as ag
     ctx = ag.Context(local)
     s = ag.TGVSolver(ctx, args.size)
     if args.shapes:
         for nm, v in json.loads(args.shapes).items():
+            if v[1] == 0:
+                continue
             s.set_launch_shape(nm, v[0], v[1], v[2], v[4] if len(v) > 4 else 1, v[5] if len(v) > 5 else (1 if len(v) > 4 and v[4] > 1 else 5))
     s.init_tgv()
     dt = s.cfl_dt(0.5)
