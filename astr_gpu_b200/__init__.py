@@ -435,17 +435,18 @@ class TGVSolver:
         self.ctx.check(self.ctx.L.astr_state_split_filter(self._h, int(on)))
 
     def autotune(self, on: bool):
-        """Per-pass launch-shape autotuning at the first RK3 step (default on above 100^3)."""
+        """Launch-shape autotuning, at the first RK3 step, of the passes that run a lane-scan kernel
+        (default on above 100^3; only boxes wider than 822 nodes, or pinned ones, have any)."""
         self.ctx.check(self.ctx.L.astr_state_autotune(self._h, int(on)))
 
     def set_launch_shape(self, pass_name: str, S: int, WPL: int, TI: int, LPW: int = 1, FPS: int = 5):
-        """Pin one pass's launch shape (disables autotuning)."""
+        """Pin one pass to its lane-scan kernel with this launch shape (disables autotuning)."""
         names = ["A", "B", "C", "A'", "B'", "F_C", "F_A"]
         self.ctx.check(self.ctx.L.astr_state_set_launch_shape(self._h, names.index(pass_name), S, WPL, TI, LPW, FPS))
 
     def launch_shapes(self) -> dict:
         """{pass: (rows per lane, warps per line, lines per CTA, tile pitch, lines per warp group,
-        fields per step)}."""
+        fields per step)}; a column solve gives its rows per chunk and 0 warps per line."""
         buf = (ctypes.c_int * 42)()
         self.ctx.check(self.ctx.L.astr_state_launch_shapes(self._h, buf))
         names = ["A", "B", "C", "A'", "B'", "F_C", "F_A"]

@@ -135,7 +135,7 @@ int pick_ti(int ntile, int dim, int WPL, int S, size_t budget = 110 * 1024) {
   return ti;
 }
 
-// Solve layouts compiled into the library (tgv_l*.cu, lines.cu).
+// Lane-scan layouts compiled into the library (tgv_l*.cu).
 const Layout kLayouts[] = {{3, 1}, {5, 1}, {9, 1}, {5, 2}, {9, 2}, {5, 4}, {9, 4}, {17, 1}};
 
 bool covers(const int64_t* shape, const int64_t* lb, int d, int64_t lo, int64_t hi) {
@@ -364,7 +364,8 @@ cudaError_t run_rhs(astr_state* st, double* q) {
   return run_pass(st, CFG_VB, a);
 }
 
-// One SSP-RK3 step (tgvsolver.F90:1037-1074): 6 passes per stage, diagnostics at stage 1.
+// One SSP-RK3 step (tgvsolver.F90:1037-1074): A, B, C, A', B' and the two filters per stage, diagnostics
+// at stage 1.
 cudaError_t run_step(astr_state* st, double dt, bool pending_at_start) {
   static const double rk[3][3] = {{1.0, 0.0, 1.0}, {0.75, 0.25, 0.25}, {1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0}};
   const int filt = st->p.filter_on;
@@ -500,7 +501,7 @@ int copy_fields(astr_state* st, double* dev, double* user, const int64_t* shape,
   return ASTR_OK;
 }
 
-// Per-pass autotuner: every compiled solve layout that covers the longest system of the pass
+// Autotuner of the passes that run a lane-scan kernel: every compiled layout that covers the longest system of the pass
 // direction with at least half of its rows used, and two or three tile widths each, timed on
 // scratch copies of the live state (the solution is not touched). Picks the fastest.
 cudaError_t autotune(astr_state* st) {
@@ -1188,7 +1189,7 @@ int astr_diagnostics(astr_state* st, double out[3]) {
 
 }  // extern "C"
 
-// ====================================================================== batched ensemble
+// ====================================================================== ensemble
 // Many independent periodic boxes of uneven sizes advanced together: an ensemble step is one CUDA
 // graph in which every box's step is a chain of its own passes, on up to ENS_BRANCHES parallel
 // branches, so the launches of small boxes run beside those of the others and no box waits for

@@ -1,5 +1,7 @@
-// Device primitives shared by every line kernel: the segmented Thomas solve and the right-hand
-// sides of the compact derivative and the compact filter, with all their closure rows.
+// A line operator's description, and the primitives of the lane-scan kernels (the passes of wide boxes
+// and of pinned launch shapes, the adjoint): the segmented Thomas solve and the right-hand sides of the
+// compact derivative and the compact filter, with all their closure rows. Everything else solves by
+// columns (colsolve.cuh).
 //
 // A line's tridiagonal system (rows r = 0..nsys-1, node = r - ext_lo) is owned by WPL warps:
 // lane `lane` of warp `part` owns the S consecutive rows of segment seg = part*32 + lane.
@@ -30,7 +32,8 @@ constexpr unsigned FULL = 0xffffffffu;
 // OP_FLUX: the compact interface flux of flux.F90 (rows are interfaces, outputs fh(-1..dim))
 enum OpKind { OP_DERIV = 0, OP_FILTER = 1, OP_EXPLICIT = 2, OP_FLUX = 3 };
 
-// One line operator (a compact_scheme of the reference plus the lane tables of its solve).
+// One line operator (a compact_scheme of the reference plus the lane tables of its solve; column
+// operators leave tab, nseg and S unset, and only they take OP_FLUX and OP_EXPLICIT).
 // Table layout (doubles), NS = 32*WPL segments of S rows, row t of segment seg:
 //   [2*(t*NS + seg)]            (ac2, ac3) pair for the forward sweep
 //   [2*S*NS + t*NS + seg]       pf, forward prefix product of -ac3 within the segment

@@ -2,17 +2,17 @@
 //
 // The reference stage (tgvsolver.F90:1037-1074) is: bchomo; rhscal = gradcal (12 line solves),
 // convection (15), qrhs=-qrhs, diffusion (pointwise sigma/qflux + 12 line solves); RK update;
-// filterq (15 line solves, x then y then z). Here one stage is six directional passes over
-// lines of directions A, B, C (a permutation of x, y, z); each pass stages TI lines of its
-// inputs in shared memory once and does every line solve that the stage needs along that
-// direction:
-//   A : filter-A of the previous stage (in place on q), dA(u,v,w,T), R  = -conv_A
-//   B : dB(u,v,w,T), R -= conv_B
-//   C : dC(u,v,w,T); sigma/qflux at every node from dA,dB (HBM) and dC (smem); writes the
-//       A and B viscous fluxes (7 fields) and keeps the C ones in smem; R += visc_C - conv_C
-//   A': R += visc_A
-//   B': R += visc_B, RK update, filter-B
-//   C'(F): filter-C
+// filterq (15 line solves, x then y then z). Here one stage is seven directional passes over
+// lines of directions A, B, C (a permutation of x, y, z):
+//   F_A: filter-A of the previous stage (in place on q; a lane-scan pass A may do it itself)
+//   A  : dA(u,v,w,T)
+//   B  : dB(u,v,w,T)
+//   C  : dC(u,v,w,T); sigma/qflux at every node from dA, dB (HBM) and dC (smem); stores the combined
+//        fluxes G = viscous - convective along A and B, keeps those along C in smem; R = D_C(G_C)
+//   A' : R += D_A(G_A)
+//   B' : R += D_B(G_B), RK update, filter-B
+//   F_C: filter-C
+// The column solves read u, v, w, T in A and B from fields that a pointwise kernel stores once.
 // Separable line filters commute, so filtering B, C then A (instead of x, y, z) changes only
 // rounding. Periodic halos are index wraps (tile loads read node dim-k for -k and k for dim+k,
 // the copies bchomo/bchomovec make); q at halo nodes of the convective flux is rebuilt from the

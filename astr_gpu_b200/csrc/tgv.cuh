@@ -28,7 +28,7 @@ struct Thermo {
 struct PassArgs {
   BoxGeo g;
   Thermo th;
-  LineOp opd, opf;          // compact derivative and filter along this pass's direction
+  LineOp opd, opf;          // lane-scan passes: derivative and filter along the pass's direction
   int dir;                  // physical direction of the lines (0 x, 1 y, 2 z)
   int dA, dB, dC;           // physical directions assigned to passes A, B, C
   int TI, LP;               // lines per CTA, tile line pitch

@@ -1,4 +1,5 @@
-// Pass kernels of the RK3 step (see tgv.cu for the pass structure). Included once per solve
+// Lane-scan kernels of the RK3 step's passes (see tgv.cu for the pass structure): pass C and filter-C of
+// boxes too wide for tgv_rows.cuh, and every pass whose launch shape is pinned. Included once per solve
 // layout (S rows per lane, WPL warps per line) by tgv_l*.cu so the layouts compile in parallel.
 //
 // Thread roles in a CTA of TI lines x WPL warps:

@@ -1,8 +1,7 @@
-"""Batched ensemble of uneven periodic boxes: stepping them together must give, box by box, the
-state of stepping each box alone with the same solve layout, and the same history. The batched
-pass kernels are separate compilations of the same code, so the compiler may contract a few
-multiply-adds differently: states agree to rounding (<= 1e-12 of each field's largest value after
-10 steps), not bitwise."""
+"""Ensemble of uneven periodic boxes against the same boxes stepped alone on the lane-scan kernels: the
+states agree to rounding (<= 1e-12 of each field's largest value after 10 steps; the ensemble runs
+column solves), and so do the histories. Against the same kernels they agree bit for bit
+(test_ensemble_graph.py)."""
 import numpy as np
 import pytest
 
@@ -15,7 +14,7 @@ PASSES = ["A", "B", "C", "A'", "B'", "F_C", "F_A"]
 
 
 def group_layout(n):
-    """Solve layout the library picks for a periodic box of n intervals (filter rows -3..n+3)."""
+    """A lane-scan layout for a periodic box of n intervals (filter rows -3..n+3)."""
     rows = n + 7
     for lim, lay in ((96, (3, 1)), (160, (5, 1)), (288, (9, 1)), (576, (9, 2)), (1152, (9, 4))):
         if rows <= lim:

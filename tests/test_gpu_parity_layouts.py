@@ -1,18 +1,19 @@
-"""Parity of every solve layout and tile form of the fused RK3 passes against the oracle.
+"""Parity of the RK3 passes against the oracle at large sizes: the column solves that run by default,
+and every layout and tile form of the lane-scan kernels.
 
 The oracle restates the reference miniapp (miniapps/tgv_solver_3d/tgvsolver.F90:994-1082; its
-own pin is the reference's golden file state.ref_128). The layouts that the autotuner selects
+own pin is the reference's golden file state.ref_128). The lane-scan layouts
 for large boxes -- (9,2) and (5,4) and (17,1) rows-per-lane x warps-per-line, 16-line tiles with
 two lines per warp group, fields streamed one at a time -- never occur at the sizes of the other
 RK3 tests, so each is pinned here and compared with the oracle directly:
 
-* 256^3, default (autotuned) shapes, 2 steps;
+* 256^3, default passes (column solves), 2 steps;
 * 256^3, every compiled layout covering the 263-row systems pinned on each pass in turn, with
   the streamed and two-lines-per-warp-group forms, 2 steps;
 * non-cubic boxes whose lines take different layouts per direction, every layout pinned on every
   pass at once (the 17-row lanes then carry padding rows past the staged halo), 3 steps;
-* 512^3 with the autotuned shapes the benchmark runs, and with each layout covering its 519-row
-  systems pinned on every pass, 1 step.
+* 512^3 with the default passes, which the benchmark runs, with a mixed set of lane-scan shapes, and
+  with each layout covering its 519-row systems pinned on every pass, 1 step.
 
 Tolerances: the conserved variables after the steps within 1e-12 of each field's largest value
 (the three momenta sharing their largest), well inside the 1e-10 of the parity target; the
@@ -189,8 +190,8 @@ def test_noncubic_every_layout_on_every_pass(ctx, dims):
     assert not bad, bad
 
 
-def _bench_shapes_512():
-    """The launch shapes the 512^3 benchmark ran with (recorded in its output line): (9,2) 8-line
+def _mixed_lane_shapes_512():
+    """The fastest lane-scan shapes at 512^3: (9,2) 8-line
     tiles for A and B, (5,4) 2-line tiles for C, (17,1) 16-line tiles with 2 lines per warp group
     and streamed fields for A', B', filter-A, (17,1) streamed for filter-C."""
     return [("A", 9, 2, 8), ("B", 9, 2, 8), ("C", 5, 4, 2), ("A'", 17, 1, 16, 2, 1), ("B'", 17, 1, 16, 2, 1),
@@ -209,14 +210,14 @@ def _host_mem_gb():
 
 
 def test_tgv512_headline_shapes_match_oracle(ctx):
-    """The benchmark's own workload: TGV 512^3, dt from CFL 0.5, one RK3 step with the autotuned
-    shapes, with the shapes of the recorded benchmark line, and with each layout covering the
+    """The benchmark's own workload: TGV 512^3, dt from CFL 0.5, one RK3 step with the default passes,
+    with the lane-scan shapes that were fastest at this size, and with each layout covering the
     519-row systems pinned on every pass; against one oracle step (about 50 GB of host memory)."""
     n = 512
     assert _host_mem_gb() >= 64, "the 512^3 oracle step needs about 50 GB of host memory"
     dt, qo, ho = _oracle_tgv(n, 1)
-    runs = [("autotuned", None, [])]
-    runs.append(("bench", False, _bench_shapes_512()))
+    runs = [("default", None, [])]
+    runs.append(("mixed lane-scan", False, _mixed_lane_shapes_512()))
     for S, W in [(17, 1), (9, 2), (5, 4)]:
         ti = 2 if W == 4 else 4
         pins = [(nm, S, W, ti, 1, 1) if nm in STREAMING else (nm, S, W, ti) for nm in PASSES]

@@ -1,9 +1,9 @@
 """The strict-parity build (-fmad=false: no multiply-add contraction, like the reference's
 gfortran build without -march) against the oracle (itself built with -ffp-contract=off).
 
-What remains between them is the solve algorithm: a segmented affine scan of the Thomas
-recurrences instead of the sequential sweep (commfunc.F90:790-813), whose rounding differs at
-the level of a few ulps per solve. One rhscal (tgvsolver.F90:962-992) of a 64^3 perturbed
+What remains between them is the solve algorithm: Thomas recurrences over chunks of rows joined by their
+carries instead of the sequential sweep (commfunc.F90:790-813), with the weights of converged rows
+folded into the stencil's, whose rounding differs at the level of a few ulps per solve. One rhscal (tgvsolver.F90:962-992) of a 64^3 perturbed
 state is compared field by field; each field's error is scaled by max(|R_m|_inf, p0/dx), the
 rounding floor of differentiating the O(p0) pressure (p0 = 1/(gamma M^2) = 71.4) at spacing
 dx. The same comparison of the default (contracting) build is printed beside it."""
