@@ -5,7 +5,7 @@
 // of u, v, w, T 1.82 (5350), R += D(G) 3.17 (5110), flux + update + filter 5.86 (4300 on the mean of the
 // stages); the lane-scan forms of tgv_kernels.cuh took 3.0, 3.97, 4.22 and 9.03. Registers hold the
 // tile, so 16 warps per SM are resident: load latency and the solve's two barriers bound it, not the
-// FP64 pipe (12-22 % busy).
+// FP64 pipe (12-24 % busy).
 //
 // Derivative and filter use the same chunks of rows: the derivative's system (nodes -1..N+1) is
 // embedded in the filter's (nodes -3..N+3) with identity rows, so the solution of the flux derivative

@@ -10,8 +10,8 @@
 //
 // 512^3 on a B200, ms per launch (GB/s of the fields read and written): pass C 9.74 -> 7.6 (4000), the
 // filter 2.98 -> 2.10 (5130). C is bound by latency: 16 warps per SM (128 registers, 85 KB of tiles)
-// wait at the solves' barriers (30 % of the stalls) and for the flux loop's loads (25 %); the FP64 pipe
-// is 20 % busy.
+// wait for the flux loop's loads (25 % of their cycles) and at the solves' barriers (23 %); the FP64 pipe
+// is 20 % busy (256^3).
 //
 // Bank conflicts: a warp's lanes run over the lines, then the fields, then the chunks. With NL = 2 (and
 // 8 lines in the filter) the pitch is 2 mod 16 doubles, so eight systems hit the even bank pairs and

@@ -671,7 +671,7 @@ def run_gradient(args, ws, rank, local):
     names = ["d/dx", "d/dy", "d/dz", "filter x", "filter y", "filter z"]
     dom = int(np.argmax(per_call))
     achieved = 16.0 * pts / (per_call[dom] * 1e-3) / 1e9
-    roof = {"kernel": f"k_line_api ({names[dom]})", "bound": "hbm", "achieved": achieved, "peak": pk,
+    roof = {"kernel": f"line operator ({names[dom]})", "bound": "hbm", "achieved": achieved, "peak": pk,
             "unit": "GB/s", "frac": achieved / pk, "traffic": None, "peak_kind": pk_kind,
             "alg_bytes_per_launch": 16.0 * pts, "ms_per_launch": per_call[dom],
             "per_call_ms": dict(zip(names, per_call))}
