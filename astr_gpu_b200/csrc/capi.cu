@@ -88,6 +88,7 @@ struct astr_ensemble {
 namespace {
 
 int fail(astr_ctx* c, int code, const std::string& msg) {
+  if (code == ASTR_ERR_CUDA || code == ASTR_ERR_NOMEM) cudaGetLastError();   // or the next launch reports it again
   if (c) c->err = msg;
   return code;
 }

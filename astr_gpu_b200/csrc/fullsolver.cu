@@ -742,6 +742,7 @@ struct astr_full {
 namespace {
 
 int ffail(astr_full* f, int code, const std::string& msg) {
+  if (code == ASTR_ERR_CUDA) cudaGetLastError();   // or the next launch reports it again
   if (f && f->ctx) astr_ctx_set_error(f->ctx, msg.c_str());
   return code;
 }
@@ -1081,6 +1082,7 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
       return ASTR_ERR_UNSUPPORTED;
     }
   if (make_colops(specs.data(), (int)specs.size(), astr_ctx_setup_stream(ctx)) != cudaSuccess) {
+    cudaGetLastError();
     astr_full_destroy(fs);
     astr_ctx_set_error(ctx, "scheme tables");
     return ASTR_ERR_CUDA;
@@ -1089,6 +1091,7 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
   // [+ f+ f- fh+ fh- (20), ssf and lshock (2) for the upwind convection]
   const size_t nf = upwind ? 74 : 52;
   if (cudaMalloc(&fs->buf, nf * (size_t)g.fs * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
     astr_full_destroy(fs);
     astr_ctx_set_error(ctx, "full-solver state allocation");
     return ASTR_ERR_NOMEM;
@@ -1105,6 +1108,7 @@ int astr_full_create(astr_ctx* ctx, const astr_params* p, astr_full** out) {
   if (cudaMalloc(&fs->partials, (size_t)fs->nparts * 3 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&fs->hist, (size_t)fs->hist_cap * 3 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&fs->counter, sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
     astr_full_destroy(fs);
     astr_ctx_set_error(ctx, "full-solver state allocation");
     return ASTR_ERR_NOMEM;

@@ -51,3 +51,23 @@ def test_context_on_another_device():
     q = _exercise(ctx1)
     assert _current_device() == 0
     np.testing.assert_array_equal(q, ref)
+
+
+def test_a_failed_call_leaves_the_next_one_alone():
+    """A box that does not fit in memory and a launch shape whose tiles do not fit in shared memory are
+    errors of those calls only."""
+    import astr_gpu_b200 as ag
+    ctx = ag.Context(0)
+    ref = _exercise(ctx)
+    for make, code in ((ag.TGVSolver, -5), (ag.FullSolver, -5)):
+        with pytest.raises(ag.AstrError) as e:
+            make(ctx, 1145)   # 400 and 650 GB
+        assert e.value.code == code
+        np.testing.assert_array_equal(_exercise(ctx), ref)
+    wide = ag.TGVSolver(ctx, 500, 16, 16)
+    wide.set_launch_shape("C", 17, 1, 16)
+    wide.init_tgv()
+    with pytest.raises(ag.AstrError) as e:
+        wide.rk3(1e-4, 1)
+    assert e.value.code == -2
+    np.testing.assert_array_equal(_exercise(ctx), ref)
