@@ -419,6 +419,15 @@ cudaError_t run_step(astr_state* st, double dt, bool pending_at_start) {
   return cudaSuccess;
 }
 
+// A step is queued: its history row, the filter along A it owes, the step counter and the time.
+void step_done(astr_state* st, double dt) {
+  st->row_key.push_back((double)st->nstep);
+  st->row_key.push_back(st->time);
+  st->pending = st->p.filter_on != 0;
+  st->nstep += 1;
+  st->time = st->time + dt;
+}
+
 int check_err(astr_state* st) {
   astr_ctx* ctx = st->ctx;
   int h = 0;
@@ -1059,29 +1068,25 @@ int astr_rk3_step(astr_state* st, double dt, int nsteps) {
   }
   for (int s = 0; s < nsteps; ++s) {
     const int variant = st->pending ? 1 : 0;
-    st->row_key.push_back((double)st->nstep);
-    st->row_key.push_back(st->time);
     if (st->use_graph) {
       if (!st->gexec[variant] || st->gdt[variant] != dt) {
         if (st->gexec[variant]) { cudaGraphExecDestroy(st->gexec[variant]); st->gexec[variant] = nullptr; }
         make_lane_tables(st);
-        cudaGraph_t graph;
+        cudaGraph_t graph = nullptr;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
         cudaError_t e = run_step(st, dt, variant == 1);
-        cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
+        const cudaError_t end = cudaStreamEndCapture(ctx->stream, &graph);
+        if (e == cudaSuccess) e = end;
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&st->gexec[variant], graph, 0);
+        if (graph) cudaGraphDestroy(graph);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "step capture");
-        if (e2 != cudaSuccess) return cuda_fail(ctx, e2, "cudaStreamEndCapture");
-        CK(cudaGraphInstantiate(&st->gexec[variant], graph, 0));
-        cudaGraphDestroy(graph);
         st->gdt[variant] = dt;
       }
       CK(cudaGraphLaunch(st->gexec[variant], ctx->stream));
     } else {
       CK(run_step(st, dt, variant == 1));
     }
-    st->pending = st->p.filter_on != 0;
-    st->nstep += 1;
-    st->time = st->time + dt;
+    step_done(st, dt);
   }
   return check_err(st);
 }
@@ -1115,14 +1120,8 @@ int astr_pass_timings(astr_state* st, double dt, int nsteps, double ms[8]) {
   PassTimer timer;
   g_timer = &timer;
   cudaError_t e = cudaSuccess;
-  for (int s = 0; s < nsteps && e == cudaSuccess; ++s) {
-    st->row_key.push_back((double)st->nstep);
-    st->row_key.push_back(st->time);
-    e = run_step(st, dt, st->pending);
-    st->pending = st->p.filter_on != 0;
-    st->nstep += 1;
-    st->time = st->time + dt;
-  }
+  for (int s = 0; s < nsteps && e == cudaSuccess; ++s)
+    if ((e = run_step(st, dt, st->pending)) == cudaSuccess) step_done(st, dt);
   g_timer = nullptr;
   if (e != cudaSuccess) return cuda_fail(ctx, e, "timed step");
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1325,23 +1324,13 @@ int astr_ensemble_step(astr_ensemble* e, const double* dt, int nsteps) {
   }
   for (int s = 0; s < nsteps; ++s) {
     const int variant = e->pending ? 1 : 0;
-    for (int b = 0; b < nbox; ++b) {
-      astr_state* st = e->boxes[b];
-      st->row_key.push_back((double)st->nstep);
-      st->row_key.push_back(st->time);
-    }
     if (!e->gexec[variant]) {
       const int rc = ens_capture(e, variant);
       if (rc) return rc;
     }
     CK(cudaGraphLaunch(e->gexec[variant], ctx->stream));
     e->pending = e->boxes[0]->p.filter_on != 0;
-    for (int b = 0; b < nbox; ++b) {
-      astr_state* st = e->boxes[b];
-      st->pending = e->pending;
-      st->nstep += 1;
-      st->time = st->time + dt[b];
-    }
+    for (int b = 0; b < nbox; ++b) step_done(e->boxes[b], dt[b]);
   }
   for (int b = 0; b < nbox; ++b) {
     int rc = check_err(e->boxes[b]);

@@ -71,3 +71,9 @@ def test_a_failed_call_leaves_the_next_one_alone():
         wide.rk3(1e-4, 1)
     assert e.value.code == -2
     np.testing.assert_array_equal(_exercise(ctx), ref)
+    # the step that failed left no row behind
+    assert wide.history().shape[0] == 0
+    wide.set_launch_shape("C", 17, 1, 2)
+    wide.rk3(1e-4, 2)
+    np.testing.assert_array_equal(wide.history()[:, 0], [0.0, 1.0])
+    assert np.isfinite(wide.history()).all()
